@@ -495,6 +495,14 @@ namespace mkb {
 //   D  in soft-failure mode, when the chunk has failed rays, the penalty rows (uncentred, value
 //      s_p sqrt(W) p_k) are loaded from the scratch slot into Y and accumulated the same way.
 // Output: gram [runs][P+1][P+1] as the normal-equation kernels write it.
+//
+// A run is cut into pieces of whole tuples (FusedPieces: about kPieceRays rays each) and the
+// pieces into at most kPieceGroups groups, from the plan alone. A piece accumulates from zero,
+// a group is the sum of its pieces and a run the sum of its groups, each in ascending order,
+// whoever computes them: one CTA takes a whole run, a group or a piece off the queue
+// (choose_items), so a run's bits do not depend on the batch it is in. With more than one item
+// per run the items leave their sums in the scratch, and the CTA that brings the last one (a
+// counter per run, no CTA waits) adds them up.
 namespace {
 
 constexpr int kFusedThreads = 128;
@@ -508,7 +516,16 @@ constexpr int kSlotDoubles = 10;
 constexpr bool kFusedDual = true;   // one two-seed sweep for rays with both rows
 constexpr int kMaxTileCols = MKB_MAX_VARIABLES / 8;                              // 8
 constexpr int kMaxTilePairs = kMaxTileCols * (kMaxTileCols + 1) / 2;             // 36
-constexpr int kMaxFusedSlots = 148 * 8;  // persistent CTAs at most (SMs x resident CTAs)
+constexpr int kMaxFusedSlots = 148 * 4;  // persistent CTAs at most (SMs x resident CTAs)
+// Pieces of a run: whole tuples, at least kPieceRays rays (more when a run would otherwise have
+// more than kMaxPieces); at most kPieceGroups groups of consecutive pieces. 512 rays are four
+// chunks (about 0.2 ms of one CTA), against some 2 us to stage a record and store a piece's sum.
+constexpr int kPieceRays = 512;
+constexpr int kMaxPieces = 64;
+constexpr int kPieceGroups = 4;
+// Items per CTA of the grid that the split aims at, and the most scratch the items' sums take
+constexpr int kItemsPerCta = 8;
+constexpr size_t kMaxPartialBytes = size_t(160) << 20;
 constexpr int kSegBatch = 8;             // tuple segments whose means are held at once
 
 // columns of a row: the P derivatives, the residual in column P, zero padding to 8
@@ -526,7 +543,8 @@ struct FusedShared {
     SharedTables tab;
     double w[kFusedThreads];      // sample weight if the ray is in the piston, else 0
     int any_pen;                  // chunk has a penalty row (soft mode)
-    int run;                      // run taken off the queue
+    int item;                     // item taken off the queue
+    int last;                     // this CTA brought the last sum of the run
     int2 tiles[kMaxTilePairs];    // (row tile, column tile) of every upper-triangle pair
 };
 
@@ -1003,13 +1021,56 @@ struct TypeTag {
     using type = T;
 };
 
+// The pieces and groups of a run (the same for every run of a launch).
+struct FusedPieces {
+    int count, groups;
+    int ray[kMaxPieces + 1];         // first ray of every piece, then the run's rays
+    int first[kPieceGroups + 1];     // first piece of every group, then the piece count
+};
+
+FusedPieces make_pieces(const TraceParams& p) {
+    FusedPieces c{};
+    int target = kPieceRays;
+    if (target < (p.rays + kMaxPieces - 1) / kMaxPieces)
+        target = (p.rays + kMaxPieces - 1) / kMaxPieces;
+    int have = 0;
+    for (int t = 0; t < p.n_tuples; ++t) {
+        const int f = t / p.L;
+        if (have == 0) c.ray[c.count++] = p.field_offset[f] + (t - f * p.L) * p.sample_count[f];
+        have += p.sample_count[f];
+        if (have >= target) have = 0;
+    }
+    c.ray[c.count] = p.rays;
+    c.groups = c.count < kPieceGroups ? c.count : kPieceGroups;
+    for (int g = 0; g <= c.groups; ++g) c.first[g] = g * c.count / c.groups;
+    return c;
+}
+
+// Items per run, 1, the groups or the pieces: the fewest that give every CTA of the grid
+// kItemsPerCta items (fewer leave the last round of the queue half empty), as long as their
+// sums fit the scratch. 512 objectives of 29 pieces on 444 CTAs: 17.5 ms with one item per run
+// (1.15 rounds of the queue), 11.0 ms with one per piece.
+int choose_items(const FusedPieces& c, int runs, int grid, size_t sum_bytes, size_t room) {
+    int items = 1;
+    for (const int n : {c.groups, c.count}) {
+        if (static_cast<int64_t>(items) * runs >= static_cast<int64_t>(kItemsPerCta) * grid) break;
+        if (sum_bytes * static_cast<size_t>(runs) * n > room) break;
+        items = n;
+    }
+    return items;
+}
+
 struct FusedArgs {
     AdjointParams ap;
     const double* records;
     double* gram;
-    double* scratch;       // [slots][slot_doubles]: penalty rows and checkpoints per CTA
+    double* scratch;       // [slots][slot_doubles]: penalty rows, checkpoints and sums per CTA
     int64_t slot_doubles;
-    int* queue;            // run counter
+    int* queue;            // item counter
+    int* done;             // [runs] items of the run that have left their sum
+    double* partial;       // [runs][items][pairs * 64] sums of the items (items > 1)
+    int items;             // items per run: 1, pc.groups or pc.count
+    FusedPieces pc;
     const int* run_mask;   // runs to process (null: all)
     const int* order;      // queue position -> run (null: identity)
     const int* split;      // device: queue positions [0, *split) and [*split, V) are two
@@ -1070,10 +1131,15 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
         sh.tiles[e] = make_int2(rem, j);
     }
     Keep* my_ck = ckpt + tid;
+    // this CTA's group and run sums, after the checkpoints in its slot
+    const int sum_size = pairs_max * 64;
+    double* group_sum = fa.scratch + (static_cast<int64_t>(blockIdx.x) + 1) * fa.slot_doubles -
+                        2 * sum_size;
+    double* run_sum = group_sum + sum_size;
     uint32_t uses = 0;
     for (;;) {
-        __syncthreads();  // the previous run's shared state is consumed
-        if (tid == 0) sh.run = atomicAdd(fa.queue, 1);
+        __syncthreads();  // the previous item's shared state is consumed
+        if (tid == 0) sh.item = atomicAdd(fa.queue, 1);
         __syncthreads();
         int lo = 0, hi = p.V;
         if (fa.split != nullptr && fa.part >= 0) {
@@ -1081,9 +1147,17 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
             lo = fa.part == 0 ? 0 : mid;
             hi = fa.part == 0 ? mid : p.V;
         }
-        if (lo + sh.run >= hi) break;
-        const int run = fa.order != nullptr ? fa.order[lo + sh.run] : lo + sh.run;
+        const int slot = sh.item / fa.items, item = sh.item - slot * fa.items;
+        if (lo + slot >= hi) break;
+        const int run = fa.order != nullptr ? fa.order[lo + slot] : lo + slot;
         if (fa.run_mask != nullptr && fa.run_mask[run] == 0) continue;
+        // the item's pieces: the run's, one group's, or one
+        const int piece0 = fa.items == 1                ? 0
+                           : fa.items == fa.pc.groups ? fa.pc.first[item]
+                                                        : item;
+        const int piece1 = fa.items == 1                ? fa.pc.count
+                           : fa.items == fa.pc.groups ? fa.pc.first[item + 1]
+                                                        : item + 1;
         // the run's variables, columns and surfaces
         const VarParams& v = fa.vt != nullptr ? fa.vt[run] : fa.ap.v;
         const int P = v.P;
@@ -1092,10 +1166,6 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
         const int pairs = ncols * (ncols + 1) / 2;
         const int S = surfaces_of(p, run);
         for (int i = tid; i < NPM * ES; i += kFusedThreads) E[i] = 0.0;  // padding stays 0
-        // the open tuple (kept identically by every thread): its index, weight, extra rows
-        int open_tuple = -1, extra = 0;
-        double open_w = 0.0;
-        for (int i = tid; i < pairs * 64; i += kFusedThreads) acc[i] = 0.0;
         if (!stage_to_shared(record, fa.records + static_cast<int64_t>(run) * p.stride,
                              static_cast<uint32_t>(p.stride * sizeof(double)), &sh.bar, uses++))
             return;
@@ -1113,7 +1183,13 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
             for (int k = tid; k < P; k += kFusedThreads)
                 aim_sensitivity(record, lay, v, k, aim_sens[k], aim_sens[MKB_MAX_VARIABLES + k]);
         __syncthreads();
-        for (int base = 0; base < p.rays; base += kFusedThreads) {
+        for (int piece = piece0; piece < piece1; ++piece) {
+        const int piece_end = fa.pc.ray[piece + 1];
+        // the open tuple (kept identically by every thread): its index, weight, extra rows
+        int open_tuple = -1, extra = 0;
+        double open_w = 0.0;
+        for (int i = tid; i < pairs * 64; i += kFusedThreads) acc[i] = 0.0;
+        for (int base = fa.pc.ray[piece]; base < piece_end; base += kFusedThreads) {
             const int q = base + tid;
             YT* row = Y + tid;  // this ray's row, column c at row[c * TS]
             for (int c = 0; c < NP; ++c) row[c * TS] = YT(0);
@@ -1122,7 +1198,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
             bool has_pen = false;
             double pen_val = 0.0, opl_val = 0.0;
             Sample smp{};
-            if (q < p.rays) {
+            if (q < piece_end) {
                 int f = 0;
                 while (f + 1 < p.F && q >= p.field_offset[f + 1]) ++f;
                 const int within = q - p.field_offset[f];
@@ -1185,14 +1261,15 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                 }
             }
             R[tid] = opl_val;
-            const double wv = (q < p.rays && in_piston(status)) ? smp.weight : 0.0;
+            const double wv = (q < piece_end && in_piston(status)) ? smp.weight : 0.0;
             const double swv = sqrt(wv);
             sh.w[tid] = wv;
             if (tid == 0) sh.any_pen = 0;
             __syncthreads();
             if (has_pen) sh.any_pen = 1;
             // ---- B: centre every tuple segment of the chunk ----
-            const int rows_here = p.rays - base < kFusedThreads ? p.rays - base : kFusedThreads;
+            const int rows_here = piece_end - base < kFusedThreads ? piece_end - base
+                                                                   : kFusedThreads;
             // Segments are the chunk's pieces of its tuples; rays are ordered by tuple (f-major,
             // then l), so segment k is tuple t0 + k and its rows follow from the plan alone.
             const int t0 = tuple_of(p, base);
@@ -1308,6 +1385,49 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                 __syncthreads();
             }
         }
+        // ---- the piece's sum into its group's, the group's into the run's (every element by
+        // the thread that owns it) ----
+        if (fa.items == fa.pc.count && fa.items > 1) continue;
+        int g = 0;
+        while (piece >= fa.pc.first[g + 1]) ++g;
+        const bool opens = piece == fa.pc.first[g], closes = piece + 1 == fa.pc.first[g + 1];
+        for (int i = tid; i < pairs * 64; i += kFusedThreads) {
+            double s = acc[i];
+            if (!opens) s = group_sum[i] + s;
+            if (!closes) {
+                group_sum[i] = s;
+            } else {
+                if (g > 0 && fa.items == 1) s = run_sum[i] + s;
+                if (fa.items == 1 && g + 1 < fa.pc.groups) run_sum[i] = s;
+                acc[i] = s;
+            }
+        }
+        }
+        if (fa.items > 1) {
+            // leave the item's sum; the CTA that brings the run's last adds them up
+            double* sums = fa.partial + static_cast<int64_t>(run) * fa.items * sum_size;
+            for (int i = tid; i < pairs * 64; i += kFusedThreads)
+                sums[static_cast<int64_t>(item) * sum_size + i] = acc[i];
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) sh.last = atomicAdd(&fa.done[run], 1) == fa.items - 1;
+            __syncthreads();
+            if (!sh.last) continue;
+            __threadfence();
+            const int per = fa.items == fa.pc.groups ? 0 : 1;  // 1: an item is one piece
+            for (int i = tid; i < pairs * 64; i += kFusedThreads) {
+                double total = 0.0;
+                for (int g = 0; g < fa.pc.groups; ++g) {
+                    const int first = per ? fa.pc.first[g] : g;
+                    const int end = per ? fa.pc.first[g + 1] : g + 1;
+                    double s = __ldcg(&sums[static_cast<int64_t>(first) * sum_size + i]);
+                    for (int k = first + 1; k < end; ++k)
+                        s += __ldcg(&sums[static_cast<int64_t>(k) * sum_size + i]);
+                    total = g == 0 ? s : total + s;
+                }
+                acc[i] = total;
+            }
+        }
         // ---- write the (P+1) x (P+1) symmetric gram ----
         const int n = P + 1;
         double* G = fa.gram + static_cast<int64_t>(run) * fa.gram_stride;
@@ -1338,16 +1458,38 @@ size_t fused_adjoint_smem(const TraceParams& tp, int P, size_t row_bytes) {
 }
 
 namespace {
+size_t tile_pairs(int P) {
+    const size_t n = static_cast<size_t>(fused_np(P) / 8);
+    return n * (n + 1) / 2;
+}
 int64_t fused_slot_doubles(int P, int S) {
-    return static_cast<int64_t>(fused_np(P) + kSlotDoubles * S) * kFusedThreads;
+    return static_cast<int64_t>(fused_np(P) + kSlotDoubles * S) * kFusedThreads +
+           2 * 64 * static_cast<int64_t>(tile_pairs(P));
+}
+// The scratch: the queue counter and the runs' item counters, the items' sums, the CTAs' slots
+// (each part 256-byte aligned).
+struct FusedScratch {
+    size_t counters, partial, slots;  // bytes of the first two, number of slots
+};
+FusedScratch fused_scratch(int runs, int P) {
+    auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t n = static_cast<size_t>(runs);
+    FusedScratch z;
+    z.counters = al((n + 64) * sizeof(int));
+    z.partial = n * kMaxPieces * tile_pairs(P) * 64 * sizeof(double);
+    if (z.partial > kMaxPartialBytes) z.partial = kMaxPartialBytes;
+    z.partial = al(z.partial);
+    z.slots = n * kMaxPieces < kMaxFusedSlots ? n * kMaxPieces : kMaxFusedSlots;
+    return z;
 }
 }  // namespace
 
-// Global scratch of the fused kernel: the queue counter, then one slot per persistent CTA with
-// its penalty rows and its checkpoints (rewritten for every chunk, so it stays in L2).
+// Global scratch of the fused kernel: the counters and the items' sums, then one slot per
+// persistent CTA with its penalty rows and its checkpoints (rewritten for every chunk, so it
+// stays in L2) and its group and run sums.
 size_t fused_scratch_bytes(int runs, int P, int S) {
-    const size_t slots = static_cast<size_t>(runs < kMaxFusedSlots ? runs : kMaxFusedSlots);
-    return 256 + slots * fused_slot_doubles(P, S) * sizeof(double);
+    const FusedScratch z = fused_scratch(runs, P);
+    return z.counters + z.partial + z.slots * fused_slot_doubles(P, S) * sizeof(double);
 }
 
 int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double* records,
@@ -1373,8 +1515,12 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
     fa.ap.rows = 0;
     fa.records = records;
     fa.gram = gram;
+    const FusedScratch z = fused_scratch(tp.V, p_max);
     fa.queue = static_cast<int*>(scratch);
-    fa.scratch = reinterpret_cast<double*>(static_cast<char*>(scratch) + 256);
+    fa.done = fa.queue + 64;
+    fa.partial = reinterpret_cast<double*>(static_cast<char*>(scratch) + z.counters);
+    fa.scratch = reinterpret_cast<double*>(static_cast<char*>(scratch) + z.counters + z.partial);
+    fa.pc = make_pieces(tp);
     fa.slot_doubles = fused_slot_doubles(p_max, tp.S);
     fa.run_mask = run_mask;
     fa.order = order;
@@ -1463,9 +1609,10 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
         return MKB_ERR_UNSUPPORTED;
     }
     int grid = sms * per_sm;
-    if (grid > kMaxFusedSlots) grid = kMaxFusedSlots;
-    if (grid > tp.V) grid = tp.V;
-    err = cudaMemsetAsync(fa.queue, 0, sizeof(int), stream);
+    if (grid > static_cast<int>(z.slots)) grid = static_cast<int>(z.slots);
+    fa.items = choose_items(fa.pc, tp.V, grid, tile_pairs(p_max) * 64 * sizeof(double), z.partial);
+    if (grid > static_cast<int64_t>(tp.V) * fa.items) grid = tp.V * fa.items;
+    err = cudaMemsetAsync(fa.queue, 0, (static_cast<size_t>(tp.V) + 64) * sizeof(int), stream);
     if (err != cudaSuccess) return cuda_status(err, "fused adjoint: clear queue");
     kernel<<<grid, kFusedThreads, smem, stream>>>(fa);
     count_launch();
