@@ -360,45 +360,73 @@ adjoint_rows_kernel(const __grid_constant__ AdjointParams ap, const double* __re
     }
 }
 
-// Piston projection of the raw dOPL/dx rows, one thread per (run, tuple, variable):
+// Piston projection of the raw dOPL/dx rows, one CTA per (run, tuple):
 // col_k = s sqrt(W_k) (col_k - mean) for rays in the piston, 0 otherwise, mean over the piston
 // rays in ascending sample order (adjoint_jacobian_cpu, src/optim/adjoint_jacobian.cpp:449).
+// All threads form the terms W_k col_k of a tile of samples (+0 outside the piston, which leaves
+// the bits of sums that start at +0), the thread of each column adds them up in order. Column P
+// carries the weights. J is read twice and written once; 48 runs of P = 29 and 14,448 rays: a
+// thread per (run, tuple, variable) that walked its column alone took 520 us, this 136 us.
+constexpr int kProjThreads = 128;
+constexpr int kProjRows = 64;           // samples per tile
+constexpr int kProjLd = kProjRows + 1;  // column stride of the terms
 template <bool kExact>
-__global__ void projection_kernel(const __grid_constant__ AdjointParams ap,
-                                  const uint8_t* __restrict__ status, double* __restrict__ J,
-                                  int64_t total) {
+__global__ void __launch_bounds__(kProjThreads)
+projection_kernel(const __grid_constant__ AdjointParams ap, const uint8_t* __restrict__ status,
+                  double* __restrict__ J, int64_t total) {
     using N = typename std::conditional<kExact, Exact64, double>::type;
+    extern __shared__ __align__(16) double term[];  // [P + 1][kProjLd]
+    __shared__ double sums[MKB_MAX_VARIABLES + 1];
     const TraceParams& p = ap.t;
-    const int64_t id = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (id >= total) return;
     const int P = ap.v.P;
-    const int var = static_cast<int>(id % P);
-    const int64_t rt = id / P;
-    const int tu = static_cast<int>(rt % p.n_tuples);
+    for (int64_t rt = blockIdx.x; rt < total; rt += gridDim.x) {
     const int64_t run = rt / p.n_tuples;
+    const int tu = static_cast<int>(rt - run * p.n_tuples);
     const int f = tu / p.L;
     const int l = tu - f * p.L;
     const int n = p.sample_count[f];
     const int64_t row0 = p.field_offset[f] + static_cast<int64_t>(l) * n;
     const uint8_t* st = status + run * p.rays + row0;
-    double* col = J + (run * P + var) * ap.rows + row0;
+    double* col0 = J + run * P * ap.rows + row0;
     const int mode = p.pupil_mode[f];
     const int M = mode == MKB_PUPIL_AXIS ? 1 : p.spokes;
     const double* w_tab = mode == MKB_PUPIL_AXIS ? p.w_axis : p.w_spoke;
     const double* rw_tab = mode == MKB_PUPIL_AXIS ? p.rw_axis : p.rw_spoke;
-    N w_ok(0.0), sum(0.0);
-    for (int k = 0; k < n; ++k)
-        if (in_piston(st[k])) w_ok += N(w_tab[k / M]);
-    const N scale = p.scale[tu];
-    if (!(value_of(w_ok) > 0.0)) {
-        for (int k = 0; k < n; ++k) col[k] = 0.0;
-        return;
+    const int tid = threadIdx.x, k_in = tid % kProjRows, c_in = tid / kProjRows;
+    constexpr int kColStep = kProjThreads / kProjRows;
+    N sum(0.0);
+    for (int base = 0; base < n; base += kProjRows) {
+        const int k = base + k_in;
+        const bool in = k < n && in_piston(st[k]);
+        const N w = in ? N(w_tab[k / M]) : N(0.0);
+        for (int c = c_in; c < P; c += kColStep)
+            term[c * kProjLd + k_in] = in ? value_of(w * N(col0[c * ap.rows + k])) : 0.0;
+        if (c_in == 0) term[P * kProjLd + k_in] = value_of(w);
+        __syncthreads();
+        if (tid <= P) {
+            const int rows = n - base < kProjRows ? n - base : kProjRows;
+            const double* t = term + tid * kProjLd;
+            for (int i = 0; i < rows; ++i) sum += N(t[i]);
+        }
+        __syncthreads();
     }
-    for (int k = 0; k < n; ++k)
-        if (in_piston(st[k])) sum += N(w_tab[k / M]) * N(col[k]);
-    const N mean = sum / w_ok;
-    for (int k = 0; k < n; ++k)
-        col[k] = in_piston(st[k]) ? value_of(scale * N(rw_tab[k / M]) * (N(col[k]) - mean)) : 0.0;
+    if (tid <= P) sums[tid] = value_of(sum);
+    __syncthreads();
+    const N w_ok = sums[P];
+    const bool valid = value_of(w_ok) > 0.0;
+    if (tid < P) sums[tid] = valid ? value_of(N(sums[tid]) / w_ok) : 0.0;
+    __syncthreads();
+    const N scale = p.scale[tu];
+    for (int k = k_in; k < n; k += kProjRows) {
+        const bool in = valid && in_piston(st[k]);
+        const N factor = scale * N(rw_tab[k / M]);
+        for (int c = c_in; c < P; c += kColStep) {
+            double* y = col0 + c * ap.rows + k;
+            *y = in ? value_of(factor * (N(*y) - N(sums[c]))) : 0.0;
+        }
+    }
+    __syncthreads();  // the means are consumed
+    }
 }
 
 // Writes x_i into a copy of the run's template record (VariableSet::apply): one CTA per run.
@@ -434,7 +462,8 @@ int launch_apply(const VarParams& vp, const RecordLayout& lay, const double* tem
     return cuda_status(cudaGetLastError(), "apply launch");
 }
 
-int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows,
+namespace {
+int launch_general_rows(const TraceParams& tp, const VarParams& vp, int64_t rows,
                         const double* records, double* J, bool exact, cudaStream_t stream) {
     AdjointParams ap;
     ap.t = tp;
@@ -450,6 +479,7 @@ int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows
     count_launch();
     return cuda_status(cudaGetLastError(), "adjoint rows launch");
 }
+}  // namespace
 
 int launch_projection(const TraceParams& tp, const VarParams& vp, int64_t rows,
                       const uint8_t* status, double* J, bool exact, cudaStream_t stream) {
@@ -457,13 +487,11 @@ int launch_projection(const TraceParams& tp, const VarParams& vp, int64_t rows,
     ap.t = tp;
     ap.v = vp;
     ap.rows = rows;
-    const int64_t total = static_cast<int64_t>(tp.V) * tp.n_tuples * vp.P;
-    const int threads = 128;
-    const int64_t blocks = (total + threads - 1) / threads;
-    if (exact)
-        projection_kernel<true><<<static_cast<unsigned>(blocks), threads, 0, stream>>>(ap, status, J, total);
-    else
-        projection_kernel<false><<<static_cast<unsigned>(blocks), threads, 0, stream>>>(ap, status, J, total);
+    const int64_t total = static_cast<int64_t>(tp.V) * tp.n_tuples;
+    const unsigned blocks = static_cast<unsigned>(total < INT32_MAX ? total : INT32_MAX);
+    const size_t smem = static_cast<size_t>(vp.P + 1) * kProjLd * sizeof(double);
+    auto kernel = exact ? projection_kernel<true> : projection_kernel<false>;
+    kernel<<<blocks, kProjThreads, smem, stream>>>(ap, status, J, total);
     count_launch();
     return cuda_status(cudaGetLastError(), "projection launch");
 }
@@ -605,12 +633,13 @@ __device__ __forceinline__ void accumulate_rows(const YT* Y, const double* R, in
     }
 }
 
-// Where the reverse sweep writes: the OPL row (seed 0) and the penalty row (seed 1).
-template <int K, class YT>
+// Where the reverse sweep writes: the OPL row (seed 0) and the penalty row (seed 1). LD: the type
+// of a column stride (rows in memory of their own: up to the rows of a run).
+template <int K, class YT, class LD = int>
 struct RowSinks {
     double factor[K];
     YT* row[K];
-    int ld[K];
+    LD ld[K];
 };
 
 template <class N, class Q, int kFeat>
@@ -782,7 +811,7 @@ __device__ void fused_forward_bulk(const TraceParams& p, const double* rec, cons
 // factor_k * dPhi_k/dx into sinks.row[k][col * ld_k]. The states and the step-local
 // quantities are in N, the adjoint arithmetic in A (N, or float for the mixed precision). One
 // out-of-line copy per K keeps the kernel's instruction footprint small.
-template <class N, class A, int K, int kFeat, class Q, class YT>
+template <class N, class A, int K, int kFeat, class Q, class YT, class LD>
 __device__ __noinline__ void fused_backward(const TraceParams& p, const VarParams& v,
                                             const double* rec, const double* mu_tab,
                                             const RecordLayout& lay, int S,
@@ -791,7 +820,7 @@ __device__ __noinline__ void fused_backward(const TraceParams& p, const VarParam
                                             int count, int image_branch, bool reached_image,
                                             bool soft_mode, const double (&so)[K],
                                             const double (&spn)[K],
-                                            const RowSinks<K, YT>& sinks,
+                                            const RowSinks<K, YT, LD>& sinks,
                                             const double* aim_sens) {
     const int L = p.L;
     const N zero(0.0);
@@ -997,7 +1026,7 @@ template <> struct FusedTypes<MixedPrecision> {
 };
 template <> struct FusedTypes<BulkPrecision> : FusedTypes<MixedPrecision> {};
 
-template <class N, int K, int kFeat>
+template <class N, int K, int kFeat, class LD>
 __device__ __forceinline__ void run_backward(const TraceParams& p, const VarParams& v,
                                              const double* rec, const double* mu_tab,
                                              const RecordLayout& lay, int S,
@@ -1007,7 +1036,8 @@ __device__ __forceinline__ void run_backward(const TraceParams& p, const VarPara
                                              int count, int image_branch, bool reached_image,
                                              bool soft_mode, const double (&so)[K],
                                              const double (&spn)[K],
-                                             const RowSinks<K, typename FusedTypes<N>::Row>& sinks,
+                                             const RowSinks<K, typename FusedTypes<N>::Row, LD>&
+                                                 sinks,
                                              const double* aim_sens) {
     using T = FusedTypes<N>;
     fused_backward<typename T::Bwd, typename T::Adj, K, kFeat>(p, v, rec, mu_tab, lay, S, f, l, smp, ck, stride_ck,
@@ -1443,7 +1473,169 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
     }
 }
 
+// ---- materialised rows from kept states -------------------------------------------------------
+// The raw rows dOPL/dx and the scaled penalty rows of adjoint_rows_kernel, traced as the fused
+// kernel traces them: persistent CTAs walk a contiguous range of 128-ray chunks (a variant's
+// record is staged once per range), the forward keeps every state and step quantity in the CTA's
+// scratch slot, and one reverse sweep carries both seeds. Every statement is that of the general
+// kernel, which keeps every fourth state in local memory and replays the steps, divisions and
+// roots included; with Exact64 the rows are the same bits. 48 objectives (P = 29, FP64, 14,448
+// rays): 2,930 us there, 640 us here.
+// Built for coaxial systems without ghost plates, an interior stop or transverse rows
+// (kept_rows_apply); those options change the sweep's statements and stay with the general kernel.
+struct RowsArgs {
+    AdjointParams ap;
+    const double* records;
+    double* J;
+    double* scratch;       // [gridDim.x][slot_doubles]
+    int64_t slot_doubles;  // [S][kSlotDoubles][T] states, then [T] for the writes of unused seeds
+    int chunks;            // of a variant
+    int64_t items;         // chunks of the launch
+};
+
+template <class N, int kFeat>
+__global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
+kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
+    const TraceParams& p = ra.ap.t;
+    const VarParams& vars = ra.ap.v;
+    __shared__ uint64_t bar;
+    __shared__ SharedTables tab;
+    extern __shared__ __align__(16) double dyn[];
+    double* record = dyn;                             // [stride]
+    double* mu_tab = record + ((p.stride + 1) & ~1);  // [S + 1][L]
+    const int tid = threadIdx.x;
+    const RecordLayout lay = layout_of(p);
+    const bool soft_mode = p.failure == MKB_FAILURE_SOFT;
+    constexpr int stride_ck = kSlotDoubles * kFusedThreads;
+    double* my_ck = ra.scratch + static_cast<int64_t>(blockIdx.x) * ra.slot_doubles + tid;
+    double* unused = my_ck + static_cast<int64_t>(p.S) * stride_ck;
+    copy_tables(p, tab);
+    const int64_t first = ra.items * blockIdx.x / gridDim.x;
+    const int64_t last = ra.items * (blockIdx.x + int64_t(1)) / gridDim.x;
+    int64_t staged = -1;
+    uint32_t uses = 0;
+    const int S = p.S;
+    for (int64_t item = first; item < last; ++item) {
+        const int64_t v = item / ra.chunks;
+        if (v != staged) {
+            if (!stage_to_shared(record, ra.records + v * p.stride,
+                                 static_cast<uint32_t>(p.stride * sizeof(double)), &bar, uses++))
+                return;
+            for (int i = tid; i < (S + 1) * p.L; i += kFusedThreads) {
+                const int s = i / p.L, l = i - s * p.L;
+                mu_tab[i] = s >= 1 && s < S ? value_of(N(record[lay.index + (s - 1) * p.L + l]) /
+                                                       N(record[lay.index + s * p.L + l]))
+                                            : 0.0;
+            }
+            __syncthreads();
+            staged = v;
+        }
+        const int q = static_cast<int>(item - v * ra.chunks) * kFusedThreads + tid;
+        if (q >= p.rays) continue;
+        int f = 0;
+        while (f + 1 < p.F && q >= p.field_offset[f + 1]) ++f;
+        const int within = q - p.field_offset[f];
+        const int l = within / p.sample_count[f];
+        const Sample smp = pupil_sample(p, tab, f, within - l * p.sample_count[f]);
+        int status, soft_first = kOk, count = 0, image_branch = 0;
+        uint64_t br_lo = 0, br_hi = 0;
+        double opl, penalty;
+        fused_forward<N, double, kFeat>(p, record, mu_tab, lay, S, f, l, smp, soft_mode, my_ck,
+                                        stride_ck, br_lo, br_hi, count, image_branch, status,
+                                        soft_first, opl, penalty);
+        const bool piston = in_piston(status);
+        const bool pen = soft_mode && soft_first != kOk;
+        if (!piston && !pen) continue;
+        // rows are the rays in order: the OPL row q, the penalty row rays + q
+        double* row = ra.J + v * vars.P * ra.ap.rows + q;
+        const double pfac =
+            pen ? value_of(N(p.pscale[f * p.L + l]) * N(smp.root_weight)) : 0.0;
+        if (__any_sync(__activemask(), piston && pen)) {
+            // a seed that the ray does not have writes where nothing reads
+            const double so[2] = {piston ? 1.0 : 0.0, 0.0};
+            const double sp[2] = {0.0, pen ? 1.0 : 0.0};
+            const RowSinks<2, double, int64_t> sinks{
+                {1.0, pfac},
+                {piston ? row : unused, pen ? row + p.rays : unused},
+                {piston ? ra.ap.rows : 0, pen ? ra.ap.rows : 0}};
+            run_backward<N, 2, kFeat>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
+                                      br_lo, br_hi, count, image_branch, piston, soft_mode, so, sp,
+                                      sinks, nullptr);
+        } else {
+            const double so[1] = {piston ? 1.0 : 0.0};
+            const double sp[1] = {pen ? 1.0 : 0.0};
+            const RowSinks<1, double, int64_t> sinks{
+                {piston ? 1.0 : pfac}, {piston ? row : row + p.rays}, {ra.ap.rows}};
+            run_backward<N, 1, kFeat>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
+                                      br_lo, br_hi, count, image_branch, piston, soft_mode, so, sp,
+                                      sinks, nullptr);
+        }
+    }
+}
+
+bool kept_rows_apply(const TraceParams& tp) {
+    return !tp.non_coaxial && tp.G == 0 && layout_of(tp).stop == 0 && !tp.transverse;
+}
+int64_t kept_rows_slot(const TraceParams& tp) {
+    return (static_cast<int64_t>(kSlotDoubles) * tp.S + 1) * kFusedThreads;
+}
+int64_t kept_rows_items(const TraceParams& tp) {
+    return static_cast<int64_t>(tp.V) * ((tp.rays + kFusedThreads - 1) / kFusedThreads);
+}
+
 }  // namespace
+
+size_t adjoint_rows_scratch_bytes(const TraceParams& tp) {
+    if (!kept_rows_apply(tp)) return 0;
+    const int64_t items = kept_rows_items(tp);
+    const int64_t slots = items < kMaxFusedSlots ? items : kMaxFusedSlots;
+    return static_cast<size_t>(slots * kept_rows_slot(tp)) * sizeof(double);
+}
+
+int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows,
+                        const double* records, double* J, bool exact, void* scratch,
+                        size_t scratch_bytes, cudaStream_t stream) {
+    if (!kept_rows_apply(tp)) return launch_general_rows(tp, vp, rows, records, J, exact, stream);
+    RowsArgs ra;
+    ra.ap.t = tp;
+    ra.ap.v = vp;
+    ra.ap.rows = rows;
+    ra.records = records;
+    ra.J = J;
+    ra.scratch = static_cast<double*>(scratch);
+    ra.slot_doubles = kept_rows_slot(tp);
+    ra.chunks = (tp.rays + kFusedThreads - 1) / kFusedThreads;
+    ra.items = kept_rows_items(tp);
+    if (ra.items == 0) return MKB_OK;
+    const int64_t slots = static_cast<int64_t>(scratch_bytes / sizeof(double)) / ra.slot_doubles;
+    if (scratch == nullptr || slots < 1) {
+        set_error("adjoint rows: scratch of %zu bytes needed", adjoint_rows_scratch_bytes(tp));
+        return MKB_ERR_WORKSPACE;
+    }
+    auto kernel = exact ? (vp.has_glass ? kept_rows_kernel<Exact64, 4> : kept_rows_kernel<Exact64, 0>)
+                        : (vp.has_glass ? kept_rows_kernel<double, 4> : kept_rows_kernel<double, 0>);
+    const size_t smem = sizeof(double) * (static_cast<size_t>((tp.stride + 1) & ~1) +
+                                          static_cast<size_t>((tp.S + 1) * tp.L));
+    int dev = 0, sms = 0, per_sm = 0;
+    int rc = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              static_cast<int>(smem)),
+                         "adjoint rows: shared memory attribute");
+    if (rc == MKB_OK) rc = cuda_status(cudaGetDevice(&dev), "adjoint rows: cudaGetDevice");
+    if (rc == MKB_OK)
+        rc = cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev),
+                         "adjoint rows: SM count");
+    if (rc == MKB_OK)
+        rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel,
+                                                                       kFusedThreads, smem),
+                         "adjoint rows: occupancy");
+    if (rc != MKB_OK) return rc;
+    int64_t grid = static_cast<int64_t>(sms) * (per_sm > 0 ? per_sm : 1);
+    if (grid > slots) grid = slots;
+    if (grid > ra.items) grid = ra.items;
+    kernel<<<static_cast<unsigned>(grid), kFusedThreads, smem, stream>>>(ra);
+    count_launch();
+    return cuda_status(cudaGetLastError(), "adjoint rows launch");
+}
 
 size_t fused_adjoint_smem(const TraceParams& tp, int P, size_t row_bytes) {
     const int NP = fused_np(P);

@@ -502,7 +502,10 @@ int mkb_adjoint_jacobian_device(const mkb_device_batch* templates, const mkb_res
     if (rc != MKB_OK) return rc;
     rc = launch_residuals(tp, records, r0, R, nullptr, status, plan->precision, stream);
     if (rc != MKB_OK) return rc;
-    rc = launch_adjoint_rows(tp, vp, R, records, J, exact, stream);
+    const size_t rec_bytes = align256(sizeof(double) * static_cast<size_t>(runs) * tp.stride);
+    rc = launch_adjoint_rows(tp, vp, R, records, J, exact,
+                             static_cast<char*>(workspace) + rec_bytes,
+                             workspace_bytes - rec_bytes, stream);
     if (rc != MKB_OK) return rc;
     return launch_projection(tp, vp, R, status, J, exact, stream);
 }

@@ -54,8 +54,12 @@ constexpr int kMaxVariantsPerCta = 8;
 int launch_apply(const VarParams& vp, const RecordLayout& lay, const double* templates,
                  int n_templates, const double* x, double* out, int runs, cudaStream_t stream,
                  RunVars rv = {});
+// scratch: adjoint_rows_scratch_bytes(tp) fill the GPU; fewer CTAs run with less (at least one
+// slot of the fused scratch)
+size_t adjoint_rows_scratch_bytes(const TraceParams& tp);
 int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows,
-                        const double* records, double* J, bool exact, cudaStream_t stream);
+                        const double* records, double* J, bool exact, void* scratch,
+                        size_t scratch_bytes, cudaStream_t stream);
 int launch_projection(const TraceParams& tp, const VarParams& vp, int64_t rows,
                       const uint8_t* status, double* J, bool exact, cudaStream_t stream);
 int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double* records,

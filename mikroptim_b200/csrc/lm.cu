@@ -591,7 +591,9 @@ LmLayout lm_layout(char* base, const LmSetup& s, int runs, const mkb_device_batc
     L.trial_merit = reinterpret_cast<double*>(take(8 * r));
     L.trial_failed = reinterpret_cast<int64_t*>(take(8 * r));
     L.trial_hard = reinterpret_cast<int64_t*>(take(8 * r));
-    L.fused_ws_bytes = s.fused ? fused_scratch_bytes(runs, s.pmax, tp.S) : 0;
+    L.fused_ws_bytes = s.fused ? fused_scratch_bytes(runs, s.pmax, tp.S)
+                       : s.fd  ? 0
+                               : adjoint_rows_scratch_bytes(tp);
     L.fused_ws = take(L.fused_ws_bytes);
     L.fd_ws_bytes = 0;
     if (s.fd) {
@@ -825,7 +827,8 @@ int phase_jacobian(const LmCall& c, const mkb_device_batch* templates,
             rc = launch_residuals(s.tp, L.records, L.r0, s.R, nullptr, L.status, s.precision,
                                   stream, RunMask{want, 1, 0});
         if (rc == MKB_OK)
-            rc = launch_adjoint_rows(s.tp, s.vp, s.R, L.records, L.J, s.exact, stream);
+            rc = launch_adjoint_rows(s.tp, s.vp, s.R, L.records, L.J, s.exact, L.fused_ws,
+                                     L.fused_ws_bytes, stream);
         if (rc == MKB_OK)
             rc = launch_projection(s.tp, s.vp, s.R, L.status, L.J, s.exact, stream);
     }

@@ -1,0 +1,46 @@
+"""The bit-exact Jacobian path at the edges of its tiles: the normal equations' chains (gram.cu:
+16-column tiles, 32-row stages), the rows from kept states (adjoint.cu: 128-ray chunks) and the
+piston projection (64-sample tiles), each equal to the oracle bit for bit."""
+
+import numpy as np
+import pytest
+import torch
+
+from mikroptim_b200 import engine, workloads
+from mikroptim_b200.batch import FAILURE_HARD, FAILURE_SOFT, ResidualLayout
+import oracle.pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("P", [1, 7, 15, 16, 31, 47, 64])
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 128, 197])
+def test_chains_equal_the_oracle(P, rows):
+    rng = np.random.default_rng(100 * P + rows)
+    J, r = rng.normal(size=(3, P, rows)), rng.normal(size=(3, rows))
+    J[:, :, rows // 2] = -0.0
+    got = engine.normal_equations_device(torch.from_numpy(J).cuda(), torch.from_numpy(r).cuda(),
+                                         True).cpu().numpy()
+    for i in range(3):
+        A, g = po.port().normal_equations(J[i], r[i])
+        assert np.array_equal(got[i, :P, :P], A) and np.array_equal(got[i, :P, P], g)
+        assert np.array_equal(got[i], got[i].T)
+
+
+@pytest.mark.parametrize("failure", [FAILURE_SOFT, FAILURE_HARD])
+@pytest.mark.parametrize("rings,spokes,glass", [
+    (1, 1, False),    # 35 rays, tuples of one ray
+    (3, 21, True),    # tuples of 63 rays
+    (4, 16, False),   # of 64
+    (5, 13, True),    # of 65; 7 rays in the last chunk
+])
+def test_rows_and_projection_equal_the_oracle(rings, spokes, glass, failure):
+    b, st, vs, x0 = workloads.objective(5, rings=rings, spokes=spokes, glass=glass,
+                                        failure=failure)
+    lay = ResidualLayout(b.topology, st)
+    J, r, s = engine.adjoint_jacobian_device(engine.DeviceSystemBatch(b), lay, b, vs, x0)
+    Jo, ro, so = po.port().adjoint_jacobian(b, lay, vs, x0, threads=8)
+    assert np.array_equal(s.cpu().numpy(), so) and np.array_equal(r.cpu().numpy(), ro)
+    J = J.cpu().numpy()
+    # bit for bit, the signs of zeros included
+    assert np.array_equal(J.view(np.int64), Jo.view(np.int64)), np.argwhere(J != Jo)[:5]
