@@ -542,8 +542,8 @@ constexpr int kFusedMinBlocks = 3;  // CTAs per SM the register budget is sized 
 // values; mu = n / n' per surface and wavelength is in a shared-memory table of the run).
 constexpr int kSlotDoubles = 10;
 constexpr bool kFusedDual = true;   // one two-seed sweep for rays with both rows
-constexpr int kMaxTileCols = MKB_MAX_VARIABLES / 8;                              // 8
-constexpr int kMaxTilePairs = kMaxTileCols * (kMaxTileCols + 1) / 2;             // 36
+constexpr int kMaxTileCols = (MKB_MAX_VARIABLES + 1 + 7) / 8;                    // 9
+constexpr int kMaxTilePairs = kMaxTileCols * (kMaxTileCols + 1) / 2;             // 45
 constexpr int kMaxFusedSlots = 148 * 4;  // persistent CTAs at most (SMs x resident CTAs)
 // Pieces of a run: whole tuples, at least kPieceRays rays (more when a run would otherwise have
 // more than kMaxPieces); at most kPieceGroups groups of consecutive pieces. 512 rays are four

@@ -43,3 +43,21 @@ def test_every_split_gives_the_bits_of_the_run_alone(variants, rings, spokes, pr
         err = np.abs(gram[v].cpu().numpy() - want) / (d[:, None] * d[None, :])
         assert err[:-1, :-1].max() <= 1e-12
         assert err.max() <= 1e-9
+
+
+@pytest.mark.parametrize("surfaces,P", [(41, 61), (43, 64)])
+def test_the_last_column_tile(surfaces, P):
+    """64 variables and the residual column are 65 columns: nine column tiles, 45 pairs."""
+    b, st, vs, x0 = workloads.sweep(2, surfaces=surfaces, wavelengths=2, rings=3, spokes=5,
+                                    precision=PRECISION_FP64)
+    assert vs.size == P
+    lay = ResidualLayout(b.topology, st)
+    db = engine.DeviceSystemBatch(b)
+    gram = engine.adjoint_normal_equations_device(db, lay, b, vs, x0).cpu().numpy()
+    J, r, _ = engine.adjoint_jacobian_device(db, lay, b, vs, x0)
+    X = torch.cat([J, r[:, None]], dim=1).cpu().numpy()
+    for v in range(2):
+        want = X[v] @ X[v].T
+        d = np.sqrt(np.maximum(np.diagonal(want), 1e-300))
+        err = np.abs(gram[v] - want) / (d[:, None] * d[None, :])  # bounds as above
+        assert err[:-1, :-1].max() <= 1e-12 and err.max() <= 1e-9
