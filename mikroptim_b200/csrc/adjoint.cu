@@ -811,7 +811,7 @@ __device__ void fused_forward_bulk(const TraceParams& p, const double* rec, cons
 // factor_k * dPhi_k/dx into sinks.row[k][col * ld_k]. The states and the step-local
 // quantities are in N, the adjoint arithmetic in A (N, or float for the mixed precision). One
 // out-of-line copy per K keeps the kernel's instruction footprint small.
-template <class N, class A, int K, int kFeat, class Q, class YT, class LD>
+template <class N, class A, int K, int kFeat, class Div, class Q, class YT, class LD>
 __device__ __noinline__ void fused_backward(const TraceParams& p, const VarParams& v,
                                             const double* rec, const double* mu_tab,
                                             const RecordLayout& lay, int S,
@@ -936,7 +936,7 @@ __device__ __noinline__ void fused_backward(const TraceParams& p, const VarParam
                                 sinks.row[m][col * sinks.ld[m]] = YT(value_of(factor[m] * value));
                         });
                 } else {
-                    refracting_step_backward_k<N, A, K>(pl, dl, tl, cj, N(idx[c * L + l]),
+                    refracting_step_backward_k<N, A, K, Div>(pl, dl, tl, cj, N(idx[c * L + l]),
                                                         N(idx[j * L + l]), next_branch, seed_opl,
                                                         seed_pen, adj, par, &cur.loc);
                 }
@@ -1026,7 +1026,7 @@ template <> struct FusedTypes<MixedPrecision> {
 };
 template <> struct FusedTypes<BulkPrecision> : FusedTypes<MixedPrecision> {};
 
-template <class N, int K, int kFeat, class LD>
+template <class N, int K, int kFeat, template <class> class Div, class LD>
 __device__ __forceinline__ void run_backward(const TraceParams& p, const VarParams& v,
                                              const double* rec, const double* mu_tab,
                                              const RecordLayout& lay, int S,
@@ -1040,7 +1040,7 @@ __device__ __forceinline__ void run_backward(const TraceParams& p, const VarPara
                                                  sinks,
                                              const double* aim_sens) {
     using T = FusedTypes<N>;
-    fused_backward<typename T::Bwd, typename T::Adj, K, kFeat>(p, v, rec, mu_tab, lay, S, f, l, smp, ck, stride_ck,
+    fused_backward<typename T::Bwd, typename T::Adj, K, kFeat, Div<typename T::Adj>>(p, v, rec, mu_tab, lay, S, f, l, smp, ck, stride_ck,
                                                         br_lo, br_hi, count, image_branch,
                                                         reached_image, soft_mode, so, spn, sinks,
                                                         aim_sens);
@@ -1263,7 +1263,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                         const double so[2] = {piston ? 1.0 : 0.0, 0.0};
                         const double sp[2] = {0.0, pen_sweep ? 1.0 : 0.0};
                         const RowSinks<2, YT> sinks{{1.0, pfac}, {row, prow}, {TS, kFusedThreads}};
-                        run_backward<N, 2, kFeat>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
+                        run_backward<N, 2, kFeat, ReciprocalDivisor>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
                                            br_hi, count, image_branch, piston, soft_mode, so, sp,
                                            sinks, aim_sens);
                     }
@@ -1273,19 +1273,19 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                         const double sp[1] = {pen_sweep ? 1.0 : 0.0};
                         const RowSinks<1, YT> sinks{{piston ? 1.0 : pfac}, {piston ? row : prow},
                                                 {piston ? TS : kFusedThreads}};
-                        run_backward<N, 1, kFeat>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
+                        run_backward<N, 1, kFeat, ReciprocalDivisor>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
                                            br_lo, br_hi, count, image_branch, piston, soft_mode,
                                            so, sp, sinks, aim_sens);
                     }
                 } else {  // both rows, one sweep each
                     const double so0[1] = {1.0}, sp0[1] = {0.0};
                     const RowSinks<1, YT> s0{{1.0}, {row}, {TS}};
-                    run_backward<N, 1, kFeat>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
+                    run_backward<N, 1, kFeat, ReciprocalDivisor>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
                                        br_hi, count, image_branch, true, soft_mode, so0, sp0, s0,
                                        aim_sens);
                     const double so1[1] = {0.0}, sp1[1] = {1.0};
                     const RowSinks<1, YT> s1{{pfac}, {prow}, {kFusedThreads}};
-                    run_backward<N, 1, kFeat>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
+                    run_backward<N, 1, kFeat, ReciprocalDivisor>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
                                        br_hi, count, image_branch, true, soft_mode, so1, sp1, s1,
                                        aim_sens);
                 }
@@ -1558,7 +1558,7 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
                 {1.0, pfac},
                 {piston ? row : unused, pen ? row + p.rays : unused},
                 {piston ? ra.ap.rows : 0, pen ? ra.ap.rows : 0}};
-            run_backward<N, 2, kFeat>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
+            run_backward<N, 2, kFeat, Divisor>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
                                       br_lo, br_hi, count, image_branch, piston, soft_mode, so, sp,
                                       sinks, nullptr);
         } else {
@@ -1566,7 +1566,7 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
             const double sp[1] = {pen ? 1.0 : 0.0};
             const RowSinks<1, double, int64_t> sinks{
                 {piston ? 1.0 : pfac}, {piston ? row : row + p.rays}, {ra.ap.rows}};
-            run_backward<N, 1, kFeat>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
+            run_backward<N, 1, kFeat, Divisor>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
                                       br_lo, br_hi, count, image_branch, piston, soft_mode, so, sp,
                                       sinks, nullptr);
         }

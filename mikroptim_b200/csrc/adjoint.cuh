@@ -90,6 +90,27 @@ struct Divisor<float> {
     __device__ __forceinline__ float div(float a) const { return a * r; }
 };
 
+// The divisor of the fused FP64 sweeps: the reciprocal, which depends on forward quantities
+// alone, is divided ahead of the adjoints' dependent chain, and a quotient on that chain is a
+// multiply and one correction by its exact remainder. With a correctly rounded reciprocal the
+// corrected quotient is the rounded one (P. Markstein, IBM J. Res. Dev. 34, 1990) except where
+// the remainder underflows, for a reciprocal of infinity (the uncorrected quotient is returned)
+// and for the sign of a zero.
+template <class A>
+struct ReciprocalDivisor {
+    A d, r;
+    __device__ __forceinline__ explicit ReciprocalDivisor(A x) : d(x), r(A(1.0) / x) {}
+    __device__ __forceinline__ A div(A a) const {
+        const double x = value_of(d), y = value_of(r), q = value_of(a) * y;
+        const double c = fma(fma(-x, q, value_of(a)), y, q);
+        return A(c == c ? c : q);
+    }
+};
+template <>
+struct ReciprocalDivisor<float> : Divisor<float> {
+    using Divisor<float>::Divisor;
+};
+
 // K adjoint vectors through one step (K seeds of the same ray: the OPL and the penalty). The
 // step-local forward quantities are recomputed in N, the adjoint arithmetic runs in A (N for
 // the FP64 paths; float on FP64 states for the mixed path). The forward recompute and the
@@ -98,7 +119,8 @@ struct Divisor<float> {
 // the result equals the single-seed sweep bit for bit.
 // `known` (optional): the step's StepLocal quantities kept by the forward pass, used instead
 // of recomputing the divisions and square roots (the values are the same).
-template <class N, class A, int K>
+// Div: the divisor of the adjoint arithmetic.
+template <class N, class A, int K, class Div = Divisor<A>>
 __device__ __forceinline__ void refracting_step_backward_k(Vec<N> p, Vec<N> d, N t, N c,
                                                            N n_before, N n_after, int branch,
                                                            const A (&seed_opl)[K],
@@ -161,7 +183,8 @@ __device__ __forceinline__ void refracting_step_backward_k(Vec<N> p, Vec<N> d, N
     const A ainv_norm = cv<A>(inv_norm), ainv = cv<A>(inv), as = cv<A>(s), as0 = cv<A>(s0);
     const A ann = cv<A>(n_after), anb = cv<A>(n_before), aB = cv<A>(B), aH = cv<A>(H);
     const A arr = cv<A>(rr), ax = cv<A>(x), ay = cv<A>(y), axd = cv<A>(xd);
-    const Divisor<A> by_2root_k(two_a * aroot_k), by_n_after(ann), by_c(ac), by_dz(ad.z);
+    const Div by_2root_k(two_a * aroot_k), by_n_after(ann), by_dz(ad.z);
+    const Divisor<A> by_c(ac);  // missed rays alone
 #pragma unroll
     for (int m = 0; m < K; ++m) {
         const Vec<A> qb_out = adj[m].p;
