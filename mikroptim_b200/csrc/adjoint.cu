@@ -533,10 +533,20 @@ namespace mkb {
 // counter per run, no CTA waits) adds them up.
 namespace {
 
-constexpr int kFusedThreads = 128;
+// One CTA of 256 threads (FP64: up to 255 registers, no spills) or two (MIXED, FP32_BULK: 128
+// registers) per SM. Against CTAs of 128 threads, three or four to an SM, the warps of a
+// scheduler are in the same phase more often and share its instruction fetches (ncu: a quarter
+// of the stalls of 128-thread CTAs were missing instructions), one accumulator and record serve
+// twice the rays, and the FP64 instances no longer spill. 128 -> 256 threads: 512 objectives
+// (FP64) 9.62 -> 9.33 ms, 2,048 uneven systems (MIXED) 21.9 -> 19.9 ms, merit and gradient of
+// 1,024 toleranced samples 17.8 -> 17.0 ms, six LM iterations of 512 uneven systems (FP64_FMA)
+// 53.5 -> 50.2 ms. 384 threads of 168 registers: 10.8 ms where 128 threads took 11.0 (FP64),
+// 24.2 where they took 21.9 (MIXED).
+constexpr int kFusedThreads = 256;
 constexpr int kFusedWarps = kFusedThreads / 32;
+constexpr int kRowsThreads = 128;   // of kept_rows_kernel: three CTAs of 168 registers per SM
+constexpr int kRowsMinBlocks = 3;   // (640 us; 256 threads took 800 us)
 constexpr int kExtraRows = 8;
-constexpr int kFusedMinBlocks = 3;  // CTAs per SM the register budget is sized for
 // Per ray and table surface c the forward pass keeps, in the CTA's scratch slot, the state
 // entering the step c -> c + 1 and that step's StepLocal quantities but mu (kSlotDoubles
 // values; mu = n / n' per surface and wavelength is in a shared-memory table of the run).
@@ -544,10 +554,11 @@ constexpr int kSlotDoubles = 10;
 constexpr bool kFusedDual = true;   // one two-seed sweep for rays with both rows
 constexpr int kMaxTileCols = (MKB_MAX_VARIABLES + 1 + 7) / 8;                    // 9
 constexpr int kMaxTilePairs = kMaxTileCols * (kMaxTileCols + 1) / 2;             // 45
-constexpr int kMaxFusedSlots = 148 * 4;  // persistent CTAs at most (SMs x resident CTAs)
+constexpr int kMaxFusedSlots = 148 * 2;  // persistent CTAs at most (SMs x resident CTAs)
+constexpr int kMaxRowsSlots = 148 * 4;   // of kept_rows_kernel
 // Pieces of a run: whole tuples, at least kPieceRays rays (more when a run would otherwise have
-// more than kMaxPieces); at most kPieceGroups groups of consecutive pieces. 512 rays are four
-// chunks (about 0.2 ms of one CTA), against some 2 us to stage a record and store a piece's sum.
+// more than kMaxPieces); at most kPieceGroups groups of consecutive pieces. 512 rays are two
+// chunks (about 0.1 ms of one CTA), against some 2 us to stage a record and store a piece's sum.
 constexpr int kPieceRays = 512;
 constexpr int kMaxPieces = 64;
 constexpr int kPieceGroups = 4;
@@ -642,7 +653,7 @@ struct RowSinks {
     LD ld[K];
 };
 
-template <class N, class Q, int kFeat>
+template <class N, class Q, int kFeat, int kT>
 __device__ void fused_forward(const TraceParams& p, const double* rec, const double* mu_tab,
                               const RecordLayout& lay, int S, int f, int l, const Sample& smp,
                               bool soft_mode, Q* ck,
@@ -675,11 +686,11 @@ __device__ void fused_forward(const TraceParams& p, const double* rec, const dou
     N n_before = idx[l];
     auto keep_state = [&](Q* q) {
         q[0] = Q(value_of(r.px));
-        q[1 * kFusedThreads] = Q(value_of(r.py));
-        q[2 * kFusedThreads] = Q(value_of(r.pz));
-        q[3 * kFusedThreads] = Q(value_of(r.dx));
-        q[4 * kFusedThreads] = Q(value_of(r.dy));
-        q[5 * kFusedThreads] = Q(value_of(r.dz));
+        q[1 * kT] = Q(value_of(r.py));
+        q[2 * kT] = Q(value_of(r.pz));
+        q[3 * kT] = Q(value_of(r.dx));
+        q[4 * kT] = Q(value_of(r.dy));
+        q[5 * kT] = Q(value_of(r.dz));
     };
     for (int s = 1; s < S; ++s) {
         const N n_after = idx[s * L + l];
@@ -694,10 +705,10 @@ __device__ void fused_forward(const TraceParams& p, const double* rec, const dou
                                           xf_at<(kFeat & 1) != 0>(rec, lay, s), sp, branch, &loc,
                                           plate ? &gd : nullptr, n_after);
         if (status != kOk) break;
-        q[6 * kFusedThreads] = Q(value_of(loc.s0));
-        q[7 * kFusedThreads] = Q(value_of(loc.s));
-        q[8 * kFusedThreads] = Q(value_of(loc.root_d));
-        q[9 * kFusedThreads] = Q(value_of(loc.root_k));
+        q[6 * kT] = Q(value_of(loc.s0));
+        q[7 * kT] = Q(value_of(loc.s));
+        q[8 * kT] = Q(value_of(loc.root_d));
+        q[9 * kT] = Q(value_of(loc.root_k));
         count = s + 1;
         if (s < 32) br_lo |= static_cast<uint64_t>(branch) << (2 * s);
         else br_hi |= static_cast<uint64_t>(branch) << (2 * (s - 32));
@@ -811,7 +822,7 @@ __device__ void fused_forward_bulk(const TraceParams& p, const double* rec, cons
 // factor_k * dPhi_k/dx into sinks.row[k][col * ld_k]. The states and the step-local
 // quantities are in N, the adjoint arithmetic in A (N, or float for the mixed precision). One
 // out-of-line copy per K keeps the kernel's instruction footprint small.
-template <class N, class A, int K, int kFeat, class Div, class Q, class YT, class LD>
+template <class N, class A, int K, int kFeat, int kT, class Div, class Q, class YT, class LD>
 __device__ __noinline__ void fused_backward(const TraceParams& p, const VarParams& v,
                                             const double* rec, const double* mu_tab,
                                             const RecordLayout& lay, int S,
@@ -876,10 +887,10 @@ __device__ __noinline__ void fused_backward(const TraceParams& p, const VarParam
     };
     auto load = [&](int c, Slot& sl) {
         const Q* q = ck + c * stride_ck;
-        sl.p = {N(q[0]), N(q[kFusedThreads]), N(q[2 * kFusedThreads])};
-        sl.d = {N(q[3 * kFusedThreads]), N(q[4 * kFusedThreads]), N(q[5 * kFusedThreads])};
-        sl.loc = {N(q[6 * kFusedThreads]), N(q[7 * kFusedThreads]), N(q[8 * kFusedThreads]),
-                  N(mu_tab[(c + 1) * L + l]), N(q[9 * kFusedThreads])};
+        sl.p = {N(q[0]), N(q[kT]), N(q[2 * kT])};
+        sl.d = {N(q[3 * kT]), N(q[4 * kT]), N(q[5 * kT])};
+        sl.loc = {N(q[6 * kT]), N(q[7 * kT]), N(q[8 * kT]),
+                  N(mu_tab[(c + 1) * L + l]), N(q[9 * kT])};
     };
     // the steps below the lowest one that writes a column feed no variable (with the aimed
     // pupil, every column takes the start's adjoint: the sweep runs to the start)
@@ -1026,7 +1037,7 @@ template <> struct FusedTypes<MixedPrecision> {
 };
 template <> struct FusedTypes<BulkPrecision> : FusedTypes<MixedPrecision> {};
 
-template <class N, int K, int kFeat, template <class> class Div, class LD>
+template <class N, int K, int kFeat, int kT, template <class> class Div, class LD>
 __device__ __forceinline__ void run_backward(const TraceParams& p, const VarParams& v,
                                              const double* rec, const double* mu_tab,
                                              const RecordLayout& lay, int S,
@@ -1040,10 +1051,9 @@ __device__ __forceinline__ void run_backward(const TraceParams& p, const VarPara
                                                  sinks,
                                              const double* aim_sens) {
     using T = FusedTypes<N>;
-    fused_backward<typename T::Bwd, typename T::Adj, K, kFeat, Div<typename T::Adj>>(p, v, rec, mu_tab, lay, S, f, l, smp, ck, stride_ck,
-                                                        br_lo, br_hi, count, image_branch,
-                                                        reached_image, soft_mode, so, spn, sinks,
-                                                        aim_sens);
+    fused_backward<typename T::Bwd, typename T::Adj, K, kFeat, kT, Div<typename T::Adj>>(
+        p, v, rec, mu_tab, lay, S, f, l, smp, ck, stride_ck, br_lo, br_hi, count, image_branch,
+        reached_image, soft_mode, so, spn, sinks, aim_sens);
 }
 
 template <class T>
@@ -1111,14 +1121,11 @@ struct FusedArgs {
     int64_t gram_stride;   // doubles per run of `gram`
 };
 
-// kWide: the instance for the runs with more than 31 variables in MIXED; their shared memory
-// (64 Gram columns) holds three CTAs per SM, so the register budget is that of three CTAs
-template <class N, int kFeat, bool kWide = false>
-__global__ void __launch_bounds__(kFusedThreads, (std::is_same<N, MixedPrecision>::value ||
-                                                  std::is_same<N, BulkPrecision>::value) &&
-                                                         !kWide
-                                                     ? 4
-                                                     : kFusedMinBlocks)
+template <class N, int kFeat>
+__global__ void __launch_bounds__(kFusedThreads, std::is_same<N, MixedPrecision>::value ||
+                                                         std::is_same<N, BulkPrecision>::value
+                                                     ? 2
+                                                     : 1)
 adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
     const TraceParams& p = fa.ap.t;
     __shared__ FusedShared sh;
@@ -1244,10 +1251,9 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                                              my_ck, stride_ck, br_lo, br_hi, count,
                                              image_branch, status, soft_first, opl, penalty);
                 else
-                    fused_forward<typename FusedTypes<N>::Fwd, Keep, kFeat>(p, record, mu_tab, lay, S, f, l, smp, soft_mode,
-                                                           my_ck, stride_ck, br_lo, br_hi, count,
-                                                           image_branch, status, soft_first, opl,
-                                                           penalty);
+                    fused_forward<typename FusedTypes<N>::Fwd, Keep, kFeat, kFusedThreads>(
+                        p, record, mu_tab, lay, S, f, l, smp, soft_mode, my_ck, stride_ck, br_lo,
+                        br_hi, count, image_branch, status, soft_first, opl, penalty);
                 const bool piston = in_piston(status);
                 has_pen = soft_mode && status != kOk;
                 const bool pen_sweep = has_pen && soft_first != kOk;
@@ -1263,9 +1269,9 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                         const double so[2] = {piston ? 1.0 : 0.0, 0.0};
                         const double sp[2] = {0.0, pen_sweep ? 1.0 : 0.0};
                         const RowSinks<2, YT> sinks{{1.0, pfac}, {row, prow}, {TS, kFusedThreads}};
-                        run_backward<N, 2, kFeat, ReciprocalDivisor>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
-                                           br_hi, count, image_branch, piston, soft_mode, so, sp,
-                                           sinks, aim_sens);
+                        run_backward<N, 2, kFeat, kFusedThreads, ReciprocalDivisor>(
+                            p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
+                            count, image_branch, piston, soft_mode, so, sp, sinks, aim_sens);
                     }
                 } else if (!(piston && pen_sweep)) {
                     if (piston || pen_sweep) {  // one row: its seed and its sink
@@ -1273,21 +1279,21 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                         const double sp[1] = {pen_sweep ? 1.0 : 0.0};
                         const RowSinks<1, YT> sinks{{piston ? 1.0 : pfac}, {piston ? row : prow},
                                                 {piston ? TS : kFusedThreads}};
-                        run_backward<N, 1, kFeat, ReciprocalDivisor>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
-                                           br_lo, br_hi, count, image_branch, piston, soft_mode,
-                                           so, sp, sinks, aim_sens);
+                        run_backward<N, 1, kFeat, kFusedThreads, ReciprocalDivisor>(
+                            p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
+                            count, image_branch, piston, soft_mode, so, sp, sinks, aim_sens);
                     }
                 } else {  // both rows, one sweep each
                     const double so0[1] = {1.0}, sp0[1] = {0.0};
                     const RowSinks<1, YT> s0{{1.0}, {row}, {TS}};
-                    run_backward<N, 1, kFeat, ReciprocalDivisor>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
-                                       br_hi, count, image_branch, true, soft_mode, so0, sp0, s0,
-                                       aim_sens);
+                    run_backward<N, 1, kFeat, kFusedThreads, ReciprocalDivisor>(
+                            p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
+                            count, image_branch, true, soft_mode, so0, sp0, s0, aim_sens);
                     const double so1[1] = {0.0}, sp1[1] = {1.0};
                     const RowSinks<1, YT> s1{{pfac}, {prow}, {kFusedThreads}};
-                    run_backward<N, 1, kFeat, ReciprocalDivisor>(p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
-                                       br_hi, count, image_branch, true, soft_mode, so1, sp1, s1,
-                                       aim_sens);
+                    run_backward<N, 1, kFeat, kFusedThreads, ReciprocalDivisor>(
+                            p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
+                            count, image_branch, true, soft_mode, so1, sp1, s1, aim_sens);
                 }
             }
             R[tid] = opl_val;
@@ -1316,39 +1322,44 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
             };
             for (int k0 = 0; k0 < nseg; k0 += kSegBatch) {
                 const int kn = nseg - k0 < kSegBatch ? nseg - k0 : kSegBatch;
-                // B2: weight and weighted column means of each segment, four lanes per
-                // (segment, column) taking rows h, h + 4, ... (h = lane mod 4) and a two-step
-                // shuffle sum. The eight columns of a warp and the four row phases then hit
-                // 32 different banks (column stride 4 mod 32 floats).
+                // B2: weight and weighted column means of each segment, eight lanes per (segment,
+                // two columns) taking rows h, h + 8, ... (h = lane mod 8) and a three-step
+                // shuffle sum; two columns share the weights' loads and their sum. The lanes of
+                // a (half-)warp hit different banks (column stride 4 mod 32 floats, 4 mod 16
+                // doubles).
                 {
-                    const int h = lane & 3;
-                    const unsigned quad = 0xFu << (lane & ~3);
-                    for (int pr = tid >> 2; pr < kn * (P + 1); pr += kFusedThreads / 4) {
-                        const int k = pr / (P + 1), c = pr - k * (P + 1);
+                    const int h = lane & 7;
+                    const unsigned octet = 0xFFu << (lane & ~7);
+                    const int halves = (P >> 1) + 1;  // column pairs of 0 .. P
+                    for (int pr = tid >> 3; pr < kn * halves; pr += kFusedThreads / 8) {
+                        const int k = pr / halves, c0 = 2 * (pr - k * halves);
+                        const int c1 = c0 < P ? c0 + 1 : P;
                         int a, n;
                         seg_rows(k0 + k, a, n);
-                        const YT* col = Y + c * TS + a;
+                        const YT* col0 = Y + c0 * TS + a;
+                        const YT* col1 = Y + c1 * TS + a;
                         const double* rcol = R + a;
                         const double* wr = sh.w + a;
-                        double sw_sum = 0.0, sum = 0.0;
-                        if (c != P) {
-                            for (int r = h; r < n; r += 4) {
-                                sw_sum += wr[r];
-                                sum += wr[r] * static_cast<double>(col[r]);
-                            }
-                        } else {
-                            for (int r = h; r < n; r += 4) {
-                                sw_sum += wr[r];
-                                sum += wr[r] * rcol[r];
-                            }
+                        const bool r0 = c0 == P, r1 = c1 == P;  // the residual column
+                        double sw_sum = 0.0, sum0 = 0.0, sum1 = 0.0;
+#pragma unroll 4
+                        for (int r = h; r < n; r += 8) {
+                            const double w = wr[r];
+                            sw_sum += w;
+                            sum0 += w * (r0 ? rcol[r] : static_cast<double>(col0[r]));
+                            sum1 += w * (r1 ? rcol[r] : static_cast<double>(col1[r]));
                         }
-                        sw_sum += __shfl_xor_sync(quad, sw_sum, 1);
-                        sum += __shfl_xor_sync(quad, sum, 1);
-                        sw_sum += __shfl_xor_sync(quad, sw_sum, 2);
-                        sum += __shfl_xor_sync(quad, sum, 2);
-                        if (h == 0) {
-                            seg_mean[k * NP + c] = sw_sum > 0.0 ? sum / sw_sum : 0.0;
-                            if (c == 0) seg_w[k] = sw_sum;
+#pragma unroll
+                        for (int o = 1; o <= 4; o <<= 1) {
+                            sw_sum += __shfl_xor_sync(octet, sw_sum, o);
+                            sum0 += __shfl_xor_sync(octet, sum0, o);
+                            sum1 += __shfl_xor_sync(octet, sum1, o);
+                        }
+                        if (h < 2) {
+                            const double sum = h == 0 ? sum0 : sum1;
+                            seg_mean[k * NP + (h == 0 ? c0 : c1)] =
+                                sw_sum > 0.0 ? sum / sw_sum : 0.0;
+                            if (h == 0 && c0 == 0) seg_w[k] = sw_sum;
                         }
                     }
                 }
@@ -1494,7 +1505,7 @@ struct RowsArgs {
 };
 
 template <class N, int kFeat>
-__global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
+__global__ void __launch_bounds__(kRowsThreads, kRowsMinBlocks)
 kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
     const TraceParams& p = ra.ap.t;
     const VarParams& vars = ra.ap.v;
@@ -1506,7 +1517,7 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
     const int tid = threadIdx.x;
     const RecordLayout lay = layout_of(p);
     const bool soft_mode = p.failure == MKB_FAILURE_SOFT;
-    constexpr int stride_ck = kSlotDoubles * kFusedThreads;
+    constexpr int stride_ck = kSlotDoubles * kRowsThreads;
     double* my_ck = ra.scratch + static_cast<int64_t>(blockIdx.x) * ra.slot_doubles + tid;
     double* unused = my_ck + static_cast<int64_t>(p.S) * stride_ck;
     copy_tables(p, tab);
@@ -1521,7 +1532,7 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
             if (!stage_to_shared(record, ra.records + v * p.stride,
                                  static_cast<uint32_t>(p.stride * sizeof(double)), &bar, uses++))
                 return;
-            for (int i = tid; i < (S + 1) * p.L; i += kFusedThreads) {
+            for (int i = tid; i < (S + 1) * p.L; i += kRowsThreads) {
                 const int s = i / p.L, l = i - s * p.L;
                 mu_tab[i] = s >= 1 && s < S ? value_of(N(record[lay.index + (s - 1) * p.L + l]) /
                                                        N(record[lay.index + s * p.L + l]))
@@ -1530,7 +1541,7 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
             __syncthreads();
             staged = v;
         }
-        const int q = static_cast<int>(item - v * ra.chunks) * kFusedThreads + tid;
+        const int q = static_cast<int>(item - v * ra.chunks) * kRowsThreads + tid;
         if (q >= p.rays) continue;
         int f = 0;
         while (f + 1 < p.F && q >= p.field_offset[f + 1]) ++f;
@@ -1540,9 +1551,10 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
         int status, soft_first = kOk, count = 0, image_branch = 0;
         uint64_t br_lo = 0, br_hi = 0;
         double opl, penalty;
-        fused_forward<N, double, kFeat>(p, record, mu_tab, lay, S, f, l, smp, soft_mode, my_ck,
-                                        stride_ck, br_lo, br_hi, count, image_branch, status,
-                                        soft_first, opl, penalty);
+        fused_forward<N, double, kFeat, kRowsThreads>(p, record, mu_tab, lay, S, f, l, smp, soft_mode,
+                                                      my_ck, stride_ck, br_lo, br_hi, count,
+                                                      image_branch, status, soft_first, opl,
+                                                      penalty);
         const bool piston = in_piston(status);
         const bool pen = soft_mode && soft_first != kOk;
         if (!piston && !pen) continue;
@@ -1558,7 +1570,7 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
                 {1.0, pfac},
                 {piston ? row : unused, pen ? row + p.rays : unused},
                 {piston ? ra.ap.rows : 0, pen ? ra.ap.rows : 0}};
-            run_backward<N, 2, kFeat, Divisor>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
+            run_backward<N, 2, kFeat, kRowsThreads, Divisor>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
                                       br_lo, br_hi, count, image_branch, piston, soft_mode, so, sp,
                                       sinks, nullptr);
         } else {
@@ -1566,7 +1578,7 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
             const double sp[1] = {pen ? 1.0 : 0.0};
             const RowSinks<1, double, int64_t> sinks{
                 {piston ? 1.0 : pfac}, {piston ? row : row + p.rays}, {ra.ap.rows}};
-            run_backward<N, 1, kFeat, Divisor>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
+            run_backward<N, 1, kFeat, kRowsThreads, Divisor>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
                                       br_lo, br_hi, count, image_branch, piston, soft_mode, so, sp,
                                       sinks, nullptr);
         }
@@ -1577,10 +1589,10 @@ bool kept_rows_apply(const TraceParams& tp) {
     return !tp.non_coaxial && tp.G == 0 && layout_of(tp).stop == 0 && !tp.transverse;
 }
 int64_t kept_rows_slot(const TraceParams& tp) {
-    return (static_cast<int64_t>(kSlotDoubles) * tp.S + 1) * kFusedThreads;
+    return (static_cast<int64_t>(kSlotDoubles) * tp.S + 1) * kRowsThreads;
 }
 int64_t kept_rows_items(const TraceParams& tp) {
-    return static_cast<int64_t>(tp.V) * ((tp.rays + kFusedThreads - 1) / kFusedThreads);
+    return static_cast<int64_t>(tp.V) * ((tp.rays + kRowsThreads - 1) / kRowsThreads);
 }
 
 }  // namespace
@@ -1588,7 +1600,7 @@ int64_t kept_rows_items(const TraceParams& tp) {
 size_t adjoint_rows_scratch_bytes(const TraceParams& tp) {
     if (!kept_rows_apply(tp)) return 0;
     const int64_t items = kept_rows_items(tp);
-    const int64_t slots = items < kMaxFusedSlots ? items : kMaxFusedSlots;
+    const int64_t slots = items < kMaxRowsSlots ? items : kMaxRowsSlots;
     return static_cast<size_t>(slots * kept_rows_slot(tp)) * sizeof(double);
 }
 
@@ -1604,7 +1616,7 @@ int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows
     ra.J = J;
     ra.scratch = static_cast<double*>(scratch);
     ra.slot_doubles = kept_rows_slot(tp);
-    ra.chunks = (tp.rays + kFusedThreads - 1) / kFusedThreads;
+    ra.chunks = (tp.rays + kRowsThreads - 1) / kRowsThreads;
     ra.items = kept_rows_items(tp);
     if (ra.items == 0) return MKB_OK;
     const int64_t slots = static_cast<int64_t>(scratch_bytes / sizeof(double)) / ra.slot_doubles;
@@ -1626,13 +1638,13 @@ int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows
                          "adjoint rows: SM count");
     if (rc == MKB_OK)
         rc = cuda_status(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel,
-                                                                       kFusedThreads, smem),
+                                                                       kRowsThreads, smem),
                          "adjoint rows: occupancy");
     if (rc != MKB_OK) return rc;
     int64_t grid = static_cast<int64_t>(sms) * (per_sm > 0 ? per_sm : 1);
     if (grid > slots) grid = slots;
     if (grid > ra.items) grid = ra.items;
-    kernel<<<static_cast<unsigned>(grid), kFusedThreads, smem, stream>>>(ra);
+    kernel<<<static_cast<unsigned>(grid), kRowsThreads, smem, stream>>>(ra);
     count_launch();
     return cuda_status(cudaGetLastError(), "adjoint rows launch");
 }
@@ -1771,14 +1783,7 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
         default: return adjoint_gram_kernel<BulkPrecision, 0>;
         }
     };
-    // MIXED runs with more than 31 variables (three CTAs per SM by shared memory) on the
-    // coaxial features: the instance with the three-CTA register budget
-    const bool wide = precision == MKB_PRECISION_MIXED && p_max > 31 &&
-                      (feat == 0 || feat == 2 || feat == 18);
-    const Fn kernel = wide ? (feat == 0   ? adjoint_gram_kernel<MixedPrecision, 0, true>
-                              : feat == 2 ? adjoint_gram_kernel<MixedPrecision, 2, true>
-                                          : adjoint_gram_kernel<MixedPrecision, 18, true>)
-                      : feat == 18 ? (precision == MKB_PRECISION_MIXED
+    const Fn kernel = feat == 18 ? (precision == MKB_PRECISION_MIXED
                                           ? adjoint_gram_kernel<MixedPrecision, 18>
                                       : precision == MKB_PRECISION_FP64
                                           ? adjoint_gram_kernel<Exact64, 18>
