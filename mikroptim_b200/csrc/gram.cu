@@ -19,7 +19,7 @@ namespace {
 constexpr int kGramThreads = 256;
 constexpr int kMaxCols = MKB_MAX_VARIABLES + 1;
 // exact kernel: threads, columns of a tile, rows of a staged tile, stages, column stride
-constexpr int kExactThreads = 64;
+constexpr int kExactThreads = 128;
 constexpr int kExactCols = 16;
 constexpr int kExactRows = 32;
 constexpr int kExactStages = 4;
@@ -46,13 +46,13 @@ __device__ __forceinline__ void copy_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
-// One CTA per run and pair of 16-column tiles (ta <= tb); thread (ti, tj) advances the four
-// chains of columns {ti, ti + 8} x {tj, tj + 8}, so a row costs it four shared loads for four
-// multiply-adds. Row tiles come in by 8-byte cp.async (a column starts at any multiple of R),
+// One CTA per run and pair of 16-column tiles (ta <= tb); thread (ti, tj) advances the chains of
+// column ti of the first tile with columns tj and tj + 8 of the second, three shared loads for
+// two multiply-adds. Row tiles come in by 8-byte cp.async (a column starts at any multiple of R),
 // kExactStages deep. What bounds it is the chain itself: R dependent multiply-adds. The column
 // stride of 17 16-byte units keeps the two-row loads of eight neighbouring columns on different
 // banks. 48 runs of P = 29 and 28,896 rows: one CTA per run with one chain per pair and
-// synchronous tiles took 2,975 us, this 1445 us.
+// synchronous tiles took 2,975 us, 64 threads of four chains 1,445 us, this 510 us.
 __global__ void __launch_bounds__(kExactThreads)
 gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, int P_all,
                   int64_t R, double* __restrict__ gram, const int* __restrict__ run_mask,
@@ -70,30 +70,41 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
     if (tb * kExactCols >= n) return;
     const bool diagonal = ta == tb;
     const int tid = threadIdx.x, ti = tid >> 3, tj = tid & 7;
-    const int cols = diagonal ? kExactCols : 2 * kExactCols;
-    // columns of a tile past n stay zero; the chains of those columns are not written
+    // this thread's row of every staged tile and the columns it copies; columns past n and rows
+    // past R are filled with zeros
+    constexpr int kCopies = 2 * kExactCols * kExactRows / kExactThreads;
+    constexpr int kCopyStep = kExactThreads / kExactRows;
+    const int copies = diagonal ? kCopies / 2 : kCopies;
+    const int k_in = tid & (kExactRows - 1), c_in = tid / kExactRows;
+    const double* src[kCopies];
+    bool in[kCopies];
+#pragma unroll
+    for (int i = 0; i < kCopies; ++i) {
+        const int c = c_in + i * kCopyStep;
+        const int col = c < kExactCols ? ta * kExactCols + c : tb * kExactCols + c - kExactCols;
+        in[i] = col < n && i < copies;
+        src[i] = in[i] ? column(J, r, run, col, P, stride, R) + k_in : r;
+    }
     auto load = [&](int64_t step) {
         const int64_t r0 = step * kExactRows;
-        double* dst = tile[step % kExactStages];
-        const int k = tid & (kExactRows - 1);
-        for (int c = tid / kExactRows; c < cols; c += kExactThreads / kExactRows) {
-            const int col = c < kExactCols ? ta * kExactCols + c
-                                           : tb * kExactCols + c - kExactCols;
-            const bool in = col < n && r0 + k < R;
-            const double* src = in ? column(J, r, run, col, P, stride, R) + r0 + k : r;
-            copy_async8(dst + c * kExactLd + k, src, in);
-        }
+        double* dst = tile[step % kExactStages] + c_in * kExactLd + k_in;
+        const bool row = r0 + k_in < R;
+#pragma unroll
+        for (int i = 0; i < kCopies; ++i)
+            if (i < copies)
+                copy_async8(dst + i * kCopyStep * kExactLd, in[i] && row ? src[i] + r0 : r,
+                            in[i] && row);
     };
     const int64_t steps = (R + kExactRows - 1) / kExactRows;
     for (int s = 0; s < kExactStages - 1; ++s) {
         if (s < steps) load(s);
         copy_async_commit();
     }
-    const bool mine = (!diagonal || ti <= tj) && ta * kExactCols + ti < n &&
-                      tb * kExactCols + tj < n;
+    const int p = ta * kExactCols + ti, q = tb * kExactCols + tj;  // chains (p, q), (p, q + 8)
+    const bool mine = p < n && q < n && (!diagonal || ti <= tj + 8);
     const int u_at = ti * kExactLd, v_at = (diagonal ? tj : kExactCols + tj) * kExactLd;
-    constexpr int kNext = 8 * kExactLd;  // the thread's second column of each tile
-    double a00 = 0.0, a01 = 0.0, a10 = 0.0, a11 = 0.0;
+    constexpr int kNext = 8 * kExactLd;
+    double a0 = 0.0, a1 = 0.0;
     for (int64_t step = 0; step < steps; ++step) {
         copy_async_wait<kExactStages - 2>();
         __syncthreads();  // this step's rows are here; the slot of the last one is free
@@ -104,42 +115,45 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
         const double* v = tile[step % kExactStages] + v_at;
         const int64_t left = R - step * kExactRows;
         if (left >= kExactRows) {
+            // eight rows' loads ahead of their chains
+            double2 us[2][4], v0[2][4], v1[2][4];
+            auto fetch = [&](int k, int h) {
 #pragma unroll
-            for (int k = 0; k < kExactRows; k += 2) {
-                const double2 u0 = *reinterpret_cast<const double2*>(u + k);
-                const double2 u1 = *reinterpret_cast<const double2*>(u + kNext + k);
-                const double2 v0 = *reinterpret_cast<const double2*>(v + k);
-                const double2 v1 = *reinterpret_cast<const double2*>(v + kNext + k);
-                a00 = fma(u0.x, v0.x, a00);
-                a01 = fma(u0.x, v1.x, a01);
-                a10 = fma(u1.x, v0.x, a10);
-                a11 = fma(u1.x, v1.x, a11);
-                a00 = fma(u0.y, v0.y, a00);
-                a01 = fma(u0.y, v1.y, a01);
-                a10 = fma(u1.y, v0.y, a10);
-                a11 = fma(u1.y, v1.y, a11);
+                for (int i = 0; i < 4; ++i) {
+                    us[h][i] = *reinterpret_cast<const double2*>(u + k + 2 * i);
+                    v0[h][i] = *reinterpret_cast<const double2*>(v + k + 2 * i);
+                    v1[h][i] = *reinterpret_cast<const double2*>(v + kNext + k + 2 * i);
+                }
+            };
+            fetch(0, 0);
+#pragma unroll
+            for (int k = 0; k < kExactRows; k += 8) {
+                const int h = (k >> 3) & 1;
+                if (k + 8 < kExactRows) fetch(k + 8, h ^ 1);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    a0 = fma(us[h][i].x, v0[h][i].x, a0);
+                    a1 = fma(us[h][i].x, v1[h][i].x, a1);
+                    a0 = fma(us[h][i].y, v0[h][i].y, a0);
+                    a1 = fma(us[h][i].y, v1[h][i].y, a1);
+                }
             }
         } else {
             for (int k = 0; k < left; ++k) {
-                a00 = fma(u[k], v[k], a00);
-                a01 = fma(u[k], v[kNext + k], a01);
-                a10 = fma(u[kNext + k], v[k], a10);
-                a11 = fma(u[kNext + k], v[kNext + k], a11);
+                a0 = fma(u[k], v[k], a0);
+                a1 = fma(u[k], v[kNext + k], a1);
             }
         }
     }
     if (!mine) return;
     double* g = gram + run * (stride + 1) * (stride + 1);
-    const double acc[2][2] = {{a00, a01}, {a10, a11}};
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int p = ta * kExactCols + ti + 8 * i, q = tb * kExactCols + tj + 8 * j;
-            if (p >= n || q >= n) continue;
-            g[static_cast<int64_t>(q) * n + p] = acc[i][j];
-            g[static_cast<int64_t>(p) * n + q] = acc[i][j];
-        }
+    for (int j = 0; j < 2; ++j) {
+        const int c = q + 8 * j;
+        if (c >= n || p > c) continue;
+        const double acc = j == 0 ? a0 : a1;
+        g[static_cast<int64_t>(c) * n + p] = acc;
+        g[static_cast<int64_t>(p) * n + c] = acc;
     }
 }
 
