@@ -1088,7 +1088,7 @@ FusedPieces make_pieces(const TraceParams& p) {
 
 // Items per run, 1, the groups or the pieces: the fewest that give every CTA of the grid
 // kItemsPerCta items (fewer leave the last round of the queue half empty), as long as their
-// sums fit the scratch. 512 objectives of 29 pieces on 444 CTAs: 17.5 ms with one item per run
+// sums fit the scratch. 512 objectives of 29 pieces on 444 CTAs of 128 threads: 17.5 ms with one item per run
 // (1.15 rounds of the queue), 11.0 ms with one per piece.
 int choose_items(const FusedPieces& c, int runs, int grid, size_t sum_bytes, size_t room) {
     int items = 1;
@@ -1113,9 +1113,6 @@ struct FusedArgs {
     FusedPieces pc;
     const int* run_mask;   // runs to process (null: all)
     const int* order;      // queue position -> run (null: identity)
-    const int* split;      // device: queue positions [0, *split) and [*split, V) are two
-                           // launches (runs with <= 31 and with more variables), or null
-    int part;              // 0 or 1: which of the two ranges this launch takes; -1: all
     const VarParams* vt;   // per-run variables (null: ap.v for every run)
     int p_max;             // the largest P (sizes the shared memory and the scratch slots)
     int64_t gram_stride;   // doubles per run of `gram`
@@ -1178,15 +1175,9 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
         __syncthreads();  // the previous item's shared state is consumed
         if (tid == 0) sh.item = atomicAdd(fa.queue, 1);
         __syncthreads();
-        int lo = 0, hi = p.V;
-        if (fa.split != nullptr && fa.part >= 0) {
-            const int mid = *fa.split;
-            lo = fa.part == 0 ? 0 : mid;
-            hi = fa.part == 0 ? mid : p.V;
-        }
         const int slot = sh.item / fa.items, item = sh.item - slot * fa.items;
-        if (lo + slot >= hi) break;
-        const int run = fa.order != nullptr ? fa.order[lo + slot] : lo + slot;
+        if (slot >= p.V) break;
+        const int run = fa.order != nullptr ? fa.order[slot] : slot;
         if (fa.run_mask != nullptr && fa.run_mask[run] == 0) continue;
         // the item's pieces: the run's, one group's, or one
         const int piece0 = fa.items == 1                ? 0
@@ -1699,15 +1690,14 @@ size_t fused_scratch_bytes(int runs, int P, int S) {
 int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double* records,
                         double* gram, void* scratch, size_t scratch_bytes, int precision,
                         cudaStream_t stream, const int* run_mask, RunVars rv,
-                        const int* order, const int* split, int part, int part_pmax) {
+                        const int* order) {
     if (tp.transverse) {
         set_error("fused adjoint: transverse ray-error rows have no fused adjoint (use the "
                   "materialised adjoint Jacobian or FD)");
         return MKB_ERR_UNSUPPORTED;
     }
     if (tp.V <= 0) return MKB_OK;
-    const int p_all = rv.table != nullptr ? rv.stride : vp.P;
-    const int p_max = part_pmax > 0 ? part_pmax : p_all;  // sizes this launch's shared memory
+    const int p_max = rv.table != nullptr ? rv.stride : vp.P;  // sizes the shared memory
     if (scratch == nullptr || scratch_bytes < fused_scratch_bytes(tp.V, p_max, tp.S)) {
         set_error("fused adjoint: scratch of %zu bytes needed",
                   fused_scratch_bytes(tp.V, p_max, tp.S));
@@ -1728,11 +1718,9 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
     fa.slot_doubles = fused_slot_doubles(p_max, tp.S);
     fa.run_mask = run_mask;
     fa.order = order;
-    fa.split = split;
-    fa.part = part;
     fa.vt = rv.table;
     fa.p_max = p_max;
-    fa.gram_stride = static_cast<int64_t>(p_all + 1) * (p_all + 1);
+    fa.gram_stride = static_cast<int64_t>(p_max + 1) * (p_max + 1);
     const bool float_rows =
         precision == MKB_PRECISION_MIXED || precision == MKB_PRECISION_FP32_BULK;
     const size_t smem = fused_adjoint_smem(tp, p_max, float_rows ? sizeof(float) : sizeof(double));
