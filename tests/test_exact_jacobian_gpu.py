@@ -27,6 +27,22 @@ def test_chains_equal_the_oracle(P, rows):
         assert np.array_equal(got[i], got[i].T)
 
 
+@pytest.mark.parametrize("P", [1, 4, 7, 8])
+@pytest.mark.parametrize("rows", [1, 3, 127, 128, 129, 900])
+def test_tensor_core_sums_of_few_columns(P, rows):
+    """Eight columns or fewer take one tile without staging. A sum of n products is within
+    n 2^-53 sum |a b| of the exact one in any order."""
+    rng = np.random.default_rng(100 * P + rows)
+    J, r = rng.normal(size=(3, P, rows)), rng.normal(size=(3, rows))
+    got = engine.normal_equations_device(torch.from_numpy(J).cuda(), torch.from_numpy(r).cuda(),
+                                         False).cpu().numpy()
+    X = np.concatenate([J, r[:, None]], axis=1).astype(np.longdouble)
+    want = X @ X.transpose(0, 2, 1)
+    bound = (rows + 1) * 2.0 ** -53 * (np.abs(X) @ np.abs(X).transpose(0, 2, 1))
+    assert (np.abs(got - want) <= bound).all()
+    assert np.array_equal(got, got.transpose(0, 2, 1))
+
+
 @pytest.mark.parametrize("failure", [FAILURE_SOFT, FAILURE_HARD])
 @pytest.mark.parametrize("rings,spokes,glass", [
     (1, 1, False),    # 35 rays, tuples of one ray
