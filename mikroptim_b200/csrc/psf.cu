@@ -52,15 +52,6 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// exp(-2 pi i m / M) for any m >= 0 from the half table
-__device__ __forceinline__ double2 twiddle(const double2* tw, int m, int M) {
-    m &= M - 1;
-    const int h = M >> 1;
-    if (m < h) return tw[m];
-    const double2 w = tw[m - h];
-    return make_double2(-w.x, -w.y);
-}
-
 __device__ __forceinline__ int bit_reverse(int i, int log_m) {
     return log_m == 0 ? 0 : static_cast<int>(__brev(static_cast<unsigned>(i)) >> (32 - log_m));
 }
@@ -262,45 +253,31 @@ __global__ void __launch_bounds__(kPsfThreads, 3) psf_cols_kernel(const PsfArgs 
 }
 
 // MTF cuts of tuple t (one CTA): sagittal |OTF(k, 0)| and tangential |OTF(0, k)| over OTF(0).
+// Both projections are real, so one transform of (column sums) + i (row sums) gives both spectra,
+// A = (Z_k + conj Z_(M-k)) / 2 and B = (Z_k - conj Z_(M-k)) / 2i; conj of the forward transform
+// is the OTF's, the modulus is the same. A warp per entry summing M terms spent its time on the
+// twiddles' gathers: 1,120 tuples of M = 256, 130 entries: 94 us, this 17 us.
 __global__ void __launch_bounds__(kPsfThreads) psf_mtf_kernel(const PsfArgs a) {
-    extern __shared__ double proj[];  // [2][M]: column sums, row sums
+    extern __shared__ double2 sm[];  // [M] transform, [M / 2] twiddles
     const int t = blockIdx.x, M = a.M, N = a.N;
-    double* cs = proj;
-    double* rs = proj + M;
+    double2* tws = sm + M;
+    stage_twiddles(tws, a.tw, M);
     for (int q = threadIdx.x; q < M; q += blockDim.x) {
-        cs[q] = a.colsum[static_cast<int64_t>(t) * M + q];
         const double* part = a.rowpart + static_cast<int64_t>(t) * a.tiles * M + q;
         double s = 0.0;
         for (int k = 0; k < a.tiles; ++k) s += part[static_cast<int64_t>(k) * M];
-        rs[q] = s;
+        sm[bit_reverse(q, a.log_m)] = make_double2(a.colsum[static_cast<int64_t>(t) * M + q], s);
     }
     __syncthreads();
-    __shared__ double otf0;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (warp == 0) {
-        double s = 0.0;
-        for (int q = lane; q < M; q += 32) s += cs[q];
-        for (int o = 16; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) otf0 = s;
-    }
-    __syncthreads();
-    const double z = otf0;
+    fft_shared<false>(sm, M, a.log_m, 1, tws, FromShared{});
+    const double z = sm[0].x;  // OTF(0), the sum of the PSF
     const int per = N + 1;
     double* out = a.mtf + static_cast<int64_t>(t) * 2 * per;
-    for (int job = warp; job < 2 * per; job += kPsfThreads / 32) {
-        const int cut = job / per, k = job - cut * per;
-        const double* v = cut == 0 ? cs : rs;
-        double re = 0.0, im = 0.0;
-        for (int q = lane; q < M; q += 32) {
-            const double2 w = twiddle(a.tw, k * q, M);  // exp(-i ...); the OTF uses exp(+i ...)
-            re += v[q] * w.x;
-            im -= v[q] * w.y;
-        }
-        for (int o = 16; o >= 1; o >>= 1) {
-            re += __shfl_xor_sync(0xffffffffu, re, o);
-            im += __shfl_xor_sync(0xffffffffu, im, o);
-        }
-        if (lane == 0) out[cut * per + k] = z > 0.0 ? sqrt(re * re + im * im) / z : nan("");
+    for (int k = threadIdx.x; k < per; k += blockDim.x) {
+        const double2 u = sm[k & (M - 1)], v = sm[(M - k) & (M - 1)];
+        const double ax = u.x + v.x, ay = u.y - v.y, bx = u.y + v.y, by = v.x - u.x;
+        out[k] = z > 0.0 ? 0.5 * sqrt(ax * ax + ay * ay) / z : nan("");
+        out[per + k] = z > 0.0 ? 0.5 * sqrt(bx * bx + by * by) / z : nan("");
     }
 }
 
@@ -525,7 +502,7 @@ int mkb_psf_device(int32_t tuples, int32_t grid, int32_t fft_size, const double*
     // data [C][M] and the twiddles [M / 2]
     const size_t smem_rows = sizeof(double2) * (static_cast<size_t>(C) * fft_size + fft_size / 2);
     const size_t smem_cols = smem_rows;
-    const size_t smem_mtf = sizeof(double) * 2 * static_cast<size_t>(fft_size);
+    const size_t smem_mtf = sizeof(double2) * (static_cast<size_t>(fft_size) + fft_size / 2);
     using Fn = void (*)(PsfArgs);
     Fn rows = C == 16 ? psf_rows_kernel<16> : C == 8 ? psf_rows_kernel<8>
             : C == 4 ? psf_rows_kernel<4> : C == 2 ? psf_rows_kernel<2> : psf_rows_kernel<1>;
