@@ -370,7 +370,10 @@ def check(status: int, what: str) -> None:
 
 
 def ptr(array, ctype=C.c_double):
-    """ctypes pointer to a contiguous numpy array (None for None)."""
+    """ctypes pointer to a contiguous numpy array (None for None); it keeps the array alive."""
     if array is None:
         return None
-    return array.ctypes.data_as(C.POINTER(ctype))
+    try:  # a third of data_as's time, which a small call makes five to thirteen times
+        return C.pointer(ctype.from_buffer(array))
+    except (TypeError, ValueError, BufferError):  # read-only or empty
+        return array.ctypes.data_as(C.POINTER(ctype))
