@@ -249,7 +249,7 @@ gram_dmma_kernel(const double* __restrict__ J, const double* __restrict__ r, int
 // entries (lane l: column l / 4, row l % 4), so every warp streams its own rows straight from
 // memory, 32 bytes of each column at a time, and the eight warps' sums are added in order. The
 // tiled kernel leaves seven warps idle here and waits for a tile at a time; 1,024 runs of P = 4
-// and 900 rows: 45.8 us there, 17 us here.
+// and 900 rows: 45.8 us there, 10.2 us here.
 __global__ void __launch_bounds__(kGramThreads)
 gram_one_tile_kernel(const double* __restrict__ J, const double* __restrict__ r, int P_all,
                      int64_t R, double* __restrict__ gram, const int* __restrict__ run_mask,

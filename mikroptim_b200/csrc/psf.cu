@@ -59,12 +59,15 @@ __device__ __forceinline__ int bit_reverse(int i, int log_m) {
 // In-place decimation-in-time FFT (forward, exp(-2 pi i jk/M)) of `count` sequences of length
 // M held in bit-reversed order in shared memory, element i of sequence c at a[i * count + c]
 // (sequence index fastest, so the lanes of a warp touch adjacent 16-byte words). The log2 M
-// radix-2 stages run in passes of up to four: a thread loads the 2^NS elements one butterfly
+// radix-2 stages run in passes of up to three: a thread loads the 2^NS elements one butterfly
 // group of the pass touches into registers, runs the NS stages there and stores them back, so
 // shared memory is read and written once per pass instead of once per stage.
-// kFirst: the pass reads its inputs through load(c, i) (the value at bit-reversed position i
-// of sequence c) instead of from shared memory.
-template <int NS, bool kFirst, class Load>
+// kZero > 0: the first pass of sequences whose inputs past M / 2^kZero are zero. Its inputs come
+// through load(c, i) (the value at bit-reversed position i of sequence c). Of 2^kZero consecutive
+// positions only the first can be non-zero, and a butterfly with zero copies, so the pass loads
+// every 2^kZero-th value and starts with stage kZero. The pupil's rows and columns are zero past
+// N <= M / 2. 1,120 maps of 64 x 64 to 256 x 256: rows 145 -> 128 us, columns 538 -> 527 us.
+template <int NS, int kZero, class Load>
 __device__ __forceinline__ void fft_pass(double2* a, int M, int count, int s, const double2* tw,
                                          const Load& load) {
     constexpr int R = 1 << NS;
@@ -77,9 +80,11 @@ __device__ __forceinline__ void fft_pass(double2* a, int M, int count, int s, co
         double2 x[R];
 #pragma unroll
         for (int k = 0; k < R; ++k)
-            x[k] = kFirst ? load(c, base + k * h0) : a[(base + k * h0) * count + c];
+            if constexpr (kZero == 0) x[k] = a[(base + k * h0) * count + c];
+            else if (k % (1 << kZero) == 0) x[k] = load(c, base + k);
+            else x[k] = x[k & ~((1 << kZero) - 1)];
 #pragma unroll
-        for (int j = 0; j < NS; ++j) {
+        for (int j = kZero; j < NS; ++j) {
             const int hj = 1 << j;
             const int step = M >> (s + j + 1);
 #pragma unroll
@@ -99,41 +104,35 @@ __device__ __forceinline__ void fft_pass(double2* a, int M, int count, int s, co
     __syncthreads();
 }
 
-struct FromShared {
-    __device__ double2 operator()(int, int) const { return make_double2(0.0, 0.0); }
-};
-
-// The whole transform in passes of at most kPassStages radix-2 stages (2^kPassStages values
-// per thread in registers); the first pass takes its inputs from load (kFirst) or shared memory.
+// The transform in passes of at most kPassStages radix-2 stages (2^kPassStages values per thread
+// in registers).
 constexpr int kPassStages = 3;
 
-template <bool kFirst, class Load>
+template <int kZero, class Load>
 __device__ __forceinline__ void fft_pass_n(int n, double2* a, int M, int count, int s,
                                            const double2* tw, const Load& load) {
     switch (n) {
-    case 1: fft_pass<1, kFirst>(a, M, count, s, tw, load); break;
-    case 2: fft_pass<2, kFirst>(a, M, count, s, tw, load); break;
-    default:
-        if constexpr (kPassStages >= 4) {
-            if (n == 4) {
-                fft_pass<(kPassStages >= 4 ? 4 : 3), kFirst>(a, M, count, s, tw, load);
-                break;
-            }
-        }
-        fft_pass<3, kFirst>(a, M, count, s, tw, load);
-        break;
+    case 1: fft_pass<1, kZero>(a, M, count, s, tw, load); break;
+    case 2: fft_pass<2, kZero>(a, M, count, s, tw, load); break;
+    default: fft_pass<3, kZero>(a, M, count, s, tw, load); break;
     }
 }
 
-template <bool kFirst, class Load>
-__device__ void fft_shared(double2* a, int M, int log_m, int count, const double2* tw,
-                           const Load& load) {
+// stages s .. log_m - 1 of sequences in shared memory
+__device__ __forceinline__ void fft_shared(double2* a, int M, int log_m, int count, int s,
+                                           const double2* tw) {
+    for (; s < log_m; s += kPassStages)
+        fft_pass_n<0>(log_m - s < kPassStages ? log_m - s : kPassStages, a, M, count, s, tw, 0);
+}
+
+// the whole transform of sequences of N <= M / 2 values, read through load(c, i)
+template <class Load>
+__device__ __forceinline__ void fft_padded(double2* a, int M, int N, int log_m, int count,
+                                           const double2* tw, const Load& load) {
     const int n0 = log_m < kPassStages ? log_m : kPassStages;
-    if (n0 > 0) fft_pass_n<kFirst>(n0, a, M, count, 0, tw, load);
-    const FromShared none;
-    for (int s = n0; s < log_m; s += kPassStages)
-        fft_pass_n<false>(log_m - s < kPassStages ? log_m - s : kPassStages, a, M, count, s, tw,
-                          none);
+    if (4 * N <= M) fft_pass_n<2>(n0, a, M, count, 0, tw, load);
+    else fft_pass_n<1>(n0, a, M, count, 0, tw, load);
+    fft_shared(a, M, log_m, count, n0, tw);
 }
 
 // the twiddle table into shared memory (read by every butterfly)
@@ -147,6 +146,15 @@ __global__ void psf_twiddle_kernel(double2* tw, int M) {
     double s, c;
     sincospi(2.0 * static_cast<double>(k) / static_cast<double>(M), &s, &c);
     tw[k] = make_double2(c, -s);
+}
+
+// exp(2 pi i opd / lambda), 0 for NaN (outside the pupil or a failed ray)
+__device__ __noinline__ double2 pupil_value(double opd, double lambda) {
+    if (opd != opd) return make_double2(0.0, 0.0);
+    const double phase = 6.283185307179586 * (opd / lambda);
+    double s, c;
+    sincos(phase, &s, &c);
+    return make_double2(c, s);
 }
 
 // The pupil function of rows [r0, r0 + R) of tuple t, transformed along x (R = kRows, rows past
@@ -164,25 +172,14 @@ __global__ void __launch_bounds__(kPsfThreads, 3) psf_rows_kernel(const PsfArgs 
     const double* map = a.maps + (static_cast<int64_t>(t) * N + r0) * N;
     double2* tws = sm + kRows * M;
     stage_twiddles(tws, a.tw, M);
-    // the row fastest: neighbouring lanes store neighbouring elements (the position of element i
-    // is bit-reversed, so lanes along i would all store to one bank); the rows' map entries come
-    // from L1 after their first sector (1,120 maps of 64 x 64: 219 -> 145 us)
-    for (int e = threadIdx.x; e < kRows * M; e += blockDim.x) {
-        const int i = e / kRows, r = e - i * kRows;
-        double2 v = make_double2(0.0, 0.0);
-        if (i < N && r0 + r < N) {
-            const double opd = map[static_cast<int64_t>(r) * N + i];
-            if (opd == opd) {  // NaN: outside the pupil or a failed ray
-                const double phase = 6.283185307179586 * (opd / lambda);
-                double s, c;
-                sincos(phase, &s, &c);
-                v = make_double2(c, s);
-            }
-        }
-        sm[bit_reverse(i, lm) * kRows + r] = v;
-    }
     __syncthreads();
-    fft_shared<false>(sm, M, lm, kRows, tws, FromShared{});
+    // every value of the pupil function is wanted once, by the first pass
+    auto load = [&](int r, int i) {
+        const int j = bit_reverse(i, lm);
+        return j < N && r0 + r < N ? pupil_value(map[static_cast<int64_t>(r) * N + j], lambda)
+                                   : make_double2(0.0, 0.0);
+    };
+    fft_padded(sm, M, N, lm, kRows, tws, load);
     const int R = min(kRows, N - r0);
     double2* out = a.spec + static_cast<int64_t>(t) * M * N + r0;
     for (int e = threadIdx.x; e < kRows * M; e += blockDim.x) {
@@ -212,7 +209,7 @@ __global__ void __launch_bounds__(kPsfThreads, 3) psf_cols_kernel(const PsfArgs 
         const int j = bit_reverse(i, lm);
         return j < N ? in[c * N + j] : make_double2(0.0, 0.0);
     };
-    fft_shared<true>(sm, M, lm, C, tws, load);
+    fft_padded(sm, M, N, lm, C, tws, load);
     const mkb_psf_pupil_params p = a.params[t];
     double* psf = a.psf + static_cast<int64_t>(t) * M * M;
     double* part = a.rowpart + (static_cast<int64_t>(t) * a.tiles + tile) * M;
@@ -256,7 +253,7 @@ __global__ void __launch_bounds__(kPsfThreads, 3) psf_cols_kernel(const PsfArgs 
 // Both projections are real, so one transform of (column sums) + i (row sums) gives both spectra,
 // A = (Z_k + conj Z_(M-k)) / 2 and B = (Z_k - conj Z_(M-k)) / 2i; conj of the forward transform
 // is the OTF's, the modulus is the same. A warp per entry summing M terms spent its time on the
-// twiddles' gathers: 1,120 tuples of M = 256, 130 entries: 94 us, this 17 us.
+// twiddles' gathers: 1,120 tuples of M = 256, 130 entries: 94 us, this 16 us.
 __global__ void __launch_bounds__(kPsfThreads) psf_mtf_kernel(const PsfArgs a) {
     extern __shared__ double2 sm[];  // [M] transform, [M / 2] twiddles
     const int t = blockIdx.x, M = a.M, N = a.N;
@@ -269,7 +266,7 @@ __global__ void __launch_bounds__(kPsfThreads) psf_mtf_kernel(const PsfArgs a) {
         sm[bit_reverse(q, a.log_m)] = make_double2(a.colsum[static_cast<int64_t>(t) * M + q], s);
     }
     __syncthreads();
-    fft_shared<false>(sm, M, a.log_m, 1, tws, FromShared{});
+    fft_shared(sm, M, a.log_m, 1, 0, tws);
     const double z = sm[0].x;  // OTF(0), the sum of the PSF
     const int per = N + 1;
     double* out = a.mtf + static_cast<int64_t>(t) * 2 * per;
