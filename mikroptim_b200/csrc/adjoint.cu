@@ -510,7 +510,7 @@ namespace mkb {
 //      step-local quantities (warps whose rays need one row run the single-seed sweep). The row
 //      y_k = [dOPL_k/dx | OPL_k] goes to shared memory (Y, column-major, residual in column
 //      P); the scaled penalty row s_p sqrt(W) dpi/dx goes to the scratch slot;
-//   B  per tuple segment of the chunk: weighted column means (a warp per column, shuffle sums)
+//   B  per tuple segment of the chunk: weighted column means (eight lanes per two columns)
 //      and the rows centred and scaled in place by all threads, x_k = s sqrt(W_k) (y_k -
 //      mu_seg); the segment is merged into the tuple's running mean with one extra row
 //      s sqrt(W_t W_seg / (W_t + W_seg)) (mu_seg - mu_t) (Chan, Golub, LeVeque). Summed over

@@ -1,7 +1,7 @@
 // Normal equations G = [J r]^T [J r] per run (A = J^T J in the top-left P x P block,
 // g = J^T r in column P, r^T r in the corner).
 //
-// Two kernels:
+// Kernels:
 //   gram_exact_kernel -- every entry is one fused multiply-add chain over the rows in ascending
 //     order, acc = fma(u_r, v_r, acc) from acc = 0: bit-identical to the reference's
 //     normal_equations_host / gram_dot (include/mikroptim/optim/normal_equations.hpp:19,33).
@@ -52,7 +52,7 @@ __device__ __forceinline__ void copy_async_wait() {
 // kExactStages deep. What bounds it is the chain itself: R dependent multiply-adds. The column
 // stride of 17 16-byte units keeps the two-row loads of eight neighbouring columns on different
 // banks. 48 runs of P = 29 and 28,896 rows: one CTA per run with one chain per pair and
-// synchronous tiles took 2,975 us, 64 threads of four chains 1,445 us, this 510 us.
+// synchronous tiles took 2,975 us, 64 threads of four chains loaded as they go 1,445 us, this 525 us.
 __global__ void __launch_bounds__(kExactThreads)
 gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, int P_all,
                   int64_t R, double* __restrict__ gram, const int* __restrict__ run_mask,
