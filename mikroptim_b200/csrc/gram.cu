@@ -19,7 +19,7 @@ namespace {
 constexpr int kGramThreads = 256;
 constexpr int kMaxCols = MKB_MAX_VARIABLES + 1;
 // exact kernel: threads, columns of a tile, rows of a staged tile, stages, column stride
-constexpr int kExactThreads = 128;
+constexpr int kExactThreads = 64;
 constexpr int kExactCols = 16;
 constexpr int kExactRows = 32;
 constexpr int kExactStages = 4;
@@ -46,13 +46,15 @@ __device__ __forceinline__ void copy_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
-// One CTA per run and pair of 16-column tiles (ta <= tb); thread (ti, tj) advances the chains of
-// column ti of the first tile with columns tj and tj + 8 of the second, three shared loads for
-// two multiply-adds. Row tiles come in by 8-byte cp.async (a column starts at any multiple of R),
-// kExactStages deep. What bounds it is the chain itself: R dependent multiply-adds. The column
-// stride of 17 16-byte units keeps the two-row loads of eight neighbouring columns on different
-// banks. 48 runs of P = 29 and 28,896 rows: one CTA per run with one chain per pair and
-// synchronous tiles took 2,975 us, 64 threads of four chains loaded as they go 1,445 us, this 525 us.
+// One CTA per run and pair of 16-column tiles (ta <= tb); thread (ti, tj) advances the four
+// chains of columns {ti, ti + 8} x {tj, tj + 8}, so a row costs it four shared loads for four
+// multiply-adds, eight rows' loads ahead of their use. Row tiles come in by 8-byte cp.async (a
+// column starts at any multiple of R), kExactStages deep. What bounds it is the chain itself, R
+// dependent multiply-adds, and the shared loads beside it. The column stride of 17 16-byte units
+// keeps the two-row loads of eight neighbouring columns on different banks. 48 runs of P = 29 and
+// 28,896 rows: one CTA per run with one chain per pair and synchronous tiles took 2,975 us, four
+// chains a thread loaded as they go 1,445 us, 128 threads of two chains with loads ahead 525 us,
+// this 455 us.
 __global__ void __launch_bounds__(kExactThreads)
 gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, int P_all,
                   int64_t R, double* __restrict__ gram, const int* __restrict__ run_mask,
@@ -100,11 +102,12 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
         if (s < steps) load(s);
         copy_async_commit();
     }
-    const int p = ta * kExactCols + ti, q = tb * kExactCols + tj;  // chains (p, q), (p, q + 8)
-    const bool mine = p < n && q < n && (!diagonal || ti <= tj + 8);
+    // chains {p, p + 8} x {q, q + 8}; on the diagonal (p + 8, q) is the transposed pair's
+    const int p = ta * kExactCols + ti, q = tb * kExactCols + tj;
+    const bool mine = p < n && q < n && (!diagonal || ti <= tj);
     const int u_at = ti * kExactLd, v_at = (diagonal ? tj : kExactCols + tj) * kExactLd;
     constexpr int kNext = 8 * kExactLd;
-    double a0 = 0.0, a1 = 0.0;
+    double a00 = 0.0, a01 = 0.0, a10 = 0.0, a11 = 0.0;
     for (int64_t step = 0; step < steps; ++step) {
         copy_async_wait<kExactStages - 2>();
         __syncthreads();  // this step's rows are here; the slot of the last one is free
@@ -116,11 +119,12 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
         const int64_t left = R - step * kExactRows;
         if (left >= kExactRows) {
             // eight rows' loads ahead of their chains
-            double2 us[2][4], v0[2][4], v1[2][4];
+            double2 u0[2][4], u1[2][4], v0[2][4], v1[2][4];
             auto fetch = [&](int k, int h) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    us[h][i] = *reinterpret_cast<const double2*>(u + k + 2 * i);
+                    u0[h][i] = *reinterpret_cast<const double2*>(u + k + 2 * i);
+                    u1[h][i] = *reinterpret_cast<const double2*>(u + kNext + k + 2 * i);
                     v0[h][i] = *reinterpret_cast<const double2*>(v + k + 2 * i);
                     v1[h][i] = *reinterpret_cast<const double2*>(v + kNext + k + 2 * i);
                 }
@@ -132,28 +136,37 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
                 if (k + 8 < kExactRows) fetch(k + 8, h ^ 1);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    a0 = fma(us[h][i].x, v0[h][i].x, a0);
-                    a1 = fma(us[h][i].x, v1[h][i].x, a1);
-                    a0 = fma(us[h][i].y, v0[h][i].y, a0);
-                    a1 = fma(us[h][i].y, v1[h][i].y, a1);
+                    a00 = fma(u0[h][i].x, v0[h][i].x, a00);
+                    a01 = fma(u0[h][i].x, v1[h][i].x, a01);
+                    a10 = fma(u1[h][i].x, v0[h][i].x, a10);
+                    a11 = fma(u1[h][i].x, v1[h][i].x, a11);
+                    a00 = fma(u0[h][i].y, v0[h][i].y, a00);
+                    a01 = fma(u0[h][i].y, v1[h][i].y, a01);
+                    a10 = fma(u1[h][i].y, v0[h][i].y, a10);
+                    a11 = fma(u1[h][i].y, v1[h][i].y, a11);
                 }
             }
         } else {
             for (int k = 0; k < left; ++k) {
-                a0 = fma(u[k], v[k], a0);
-                a1 = fma(u[k], v[kNext + k], a1);
+                a00 = fma(u[k], v[k], a00);
+                a01 = fma(u[k], v[kNext + k], a01);
+                a10 = fma(u[kNext + k], v[k], a10);
+                a11 = fma(u[kNext + k], v[kNext + k], a11);
             }
         }
     }
     if (!mine) return;
     double* g = gram + run * (stride + 1) * (stride + 1);
+    const double acc[2][2] = {{a00, a01}, {a10, a11}};
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const int c = q + 8 * j;
-        if (c >= n || p > c) continue;
-        const double acc = j == 0 ? a0 : a1;
-        g[static_cast<int64_t>(c) * n + p] = acc;
-        g[static_cast<int64_t>(p) * n + c] = acc;
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int c = p + 8 * i, d = q + 8 * j;
+            if (c >= n || d >= n) continue;
+            g[static_cast<int64_t>(d) * n + c] = acc[i][j];
+            g[static_cast<int64_t>(c) * n + d] = acc[i][j];
+        }
     }
 }
 
