@@ -185,6 +185,43 @@ __device__ inline void dmma_8x8x4(double& d0, double& d1, double a, double b) {
                  : "d"(a), "d"(b));
 }
 
+// The sums of a run of at most eight columns (P <= 7): one 8 x 8 tile, whose two fragments are the
+// same entries (lane l: column l / 4, row l % 4), so every warp streams its own rows straight from
+// memory, 32 bytes of each column at a time, and the eight warps' sums are added in order. The
+// tiles below leave seven warps idle here and wait for a tile at a time; 1,024 runs of P = 4 and
+// 900 rows: 45.8 us there, 10.2 us here. Which way a run goes is decided by its own P alone, so
+// that its bits are the same in every batch. part: [kDmmaWarps * 64] in shared memory.
+__device__ __forceinline__ void one_tile_sums(const double* J, const double* r, int64_t run, int P,
+                                              int stride, int64_t R, double* part, double* gram) {
+    const int n = P + 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gid = lane >> 2, tig = lane & 3;
+    const bool in = gid < n;
+    const double* col = in ? column(J, r, run, gid, P, stride, R) : r;
+    // a warp's rows: 4 kUnroll at a time, the warps in turn
+    constexpr int kUnroll = 4;
+    double d0 = 0.0, d1 = 0.0;
+    for (int64_t k0 = int64_t(warp) * 4 * kUnroll; k0 < R; k0 += kDmmaWarps * 4 * kUnroll) {
+        double x[kUnroll];
+#pragma unroll
+        for (int i = 0; i < kUnroll; ++i) {
+            const int64_t k = k0 + 4 * i + tig;
+            x[i] = in && k < R ? col[k] : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < kUnroll; ++i) dmma_8x8x4(d0, d1, x[i], x[i]);
+    }
+    part[warp * 64 + gid * 8 + 2 * tig] = d0;
+    part[warp * 64 + gid * 8 + 2 * tig + 1] = d1;
+    __syncthreads();
+    if (threadIdx.x < 64) {
+        const int row = threadIdx.x >> 3, c = threadIdx.x & 7;
+        double sum = part[threadIdx.x];
+        for (int w = 1; w < kDmmaWarps; ++w) sum += part[w * 64 + threadIdx.x];
+        if (row < n && c < n) gram[run * (stride + 1) * (stride + 1) + row * n + c] = sum;
+    }
+}
+
 __global__ void __launch_bounds__(kGramThreads)
 gram_dmma_kernel(const double* __restrict__ J, const double* __restrict__ r, int P_all,
                  int64_t R, double* __restrict__ gram, const int* __restrict__ run_mask,
@@ -197,6 +234,10 @@ gram_dmma_kernel(const double* __restrict__ J, const double* __restrict__ r, int
     if (run_mask != nullptr && run_mask[run] == 0) return;
     const int P = vt != nullptr ? vt[run].P : P_all;
     const int n = P + 1;
+    if (n <= 8) {
+        one_tile_sums(J, r, run, P, stride, R, tile, gram);
+        return;
+    }
     const int T = (n + 7) / 8;
     const int pairs = T * (T + 1) / 2;
     const int warp = threadIdx.x >> 5;
@@ -258,46 +299,16 @@ gram_dmma_kernel(const double* __restrict__ J, const double* __restrict__ r, int
     }
 }
 
-// The same for at most eight columns (P <= 7): one 8 x 8 tile, whose two fragments are the same
-// entries (lane l: column l / 4, row l % 4), so every warp streams its own rows straight from
-// memory, 32 bytes of each column at a time, and the eight warps' sums are added in order. The
-// tiled kernel leaves seven warps idle here and waits for a tile at a time; 1,024 runs of P = 4
-// and 900 rows: 45.8 us there, 10.2 us here.
+// Batches of at most eight columns: the one-tile sums without the tiled kernel's shared memory and
+// registers. A wider batch's narrow runs take the same sums in gram_dmma_kernel.
 __global__ void __launch_bounds__(kGramThreads)
 gram_one_tile_kernel(const double* __restrict__ J, const double* __restrict__ r, int P_all,
                      int64_t R, double* __restrict__ gram, const int* __restrict__ run_mask,
                      const VarParams* __restrict__ vt, int stride) {
-    __shared__ double part[kDmmaWarps][64];
+    __shared__ double part[kDmmaWarps * 64];
     const int64_t run = blockIdx.x;
     if (run_mask != nullptr && run_mask[run] == 0) return;
-    const int P = vt != nullptr ? vt[run].P : P_all;
-    const int n = P + 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gid = lane >> 2, tig = lane & 3;
-    const bool in = gid < n;
-    const double* col = in ? column(J, r, run, gid, P, stride, R) : r;
-    // a warp's rows: 4 kUnroll at a time, the warps in turn
-    constexpr int kUnroll = 4;
-    double d0 = 0.0, d1 = 0.0;
-    for (int64_t k0 = int64_t(warp) * 4 * kUnroll; k0 < R; k0 += kDmmaWarps * 4 * kUnroll) {
-        double x[kUnroll];
-#pragma unroll
-        for (int i = 0; i < kUnroll; ++i) {
-            const int64_t k = k0 + 4 * i + tig;
-            x[i] = in && k < R ? col[k] : 0.0;
-        }
-#pragma unroll
-        for (int i = 0; i < kUnroll; ++i) dmma_8x8x4(d0, d1, x[i], x[i]);
-    }
-    part[warp][gid * 8 + 2 * tig] = d0;
-    part[warp][gid * 8 + 2 * tig + 1] = d1;
-    __syncthreads();
-    if (threadIdx.x < 64) {
-        const int row = threadIdx.x >> 3, c = threadIdx.x & 7;
-        double sum = part[0][threadIdx.x];
-        for (int w = 1; w < kDmmaWarps; ++w) sum += part[w][threadIdx.x];
-        if (row < n && c < n) gram[run * (stride + 1) * (stride + 1) + row * n + c] = sum;
-    }
+    one_tile_sums(J, r, run, vt != nullptr ? vt[run].P : P_all, stride, R, part, gram);
 }
 
 }  // namespace

@@ -69,6 +69,28 @@ def test_uneven_lm_equals_each_run_alone(method):
     assert np.all(together["merit"] <= together["history"][:, 0])
 
 
+def test_uneven_fd_lm_of_narrow_and_wide_runs_equals_each_run_alone():
+    """Runs of at most seven variables beside wider ones: their FD normal equations are summed in
+    the order they are summed in alone."""
+    b, st, vss, x0 = workloads.uneven(8, rings=4, spokes=8, p_min=4, p_max=11,
+                                      precision=PRECISION_FP64_FMA)
+    P = np.array([v.size for v in vss])
+    assert (P <= 7).sum() >= 2 and (P >= 8).sum() >= 2
+    lay = ResidualLayout(b.topology, st)
+    opt = engine.LmOptions(max_iterations=12, gram_exact=False, jacobian=engine.JACOBIAN_FD)
+    together = engine.optimize_lm_gpu(b, lay, vss, x0, opt)
+    for v in range(b.variants):
+        one = workloads.unpad(b, v)
+        vs_alone = type(vss[v])(one.topology, [
+            type(var)(2 if (var.type == 1 and var.surface == one.surfaces - 1) else var.type,
+                      var.surface, var.lower, var.upper, var.typical)
+            for var in vss[v].variables])
+        alone = engine.optimize_lm_gpu(one, ResidualLayout(one.topology, st), vs_alone,
+                                       x0[v][None, :], opt)
+        assert np.array_equal(together["x"][v, :P[v]], alone["x"][0]), v
+        assert together["merit"][v] == alone["merit"][0], v
+
+
 def test_uneven_fused_normal_equations_equal_each_run_alone():
     b, st, vss, x0 = _small(8, precision=0)
     lay = ResidualLayout(b.topology, st)
