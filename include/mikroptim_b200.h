@@ -330,9 +330,14 @@ int mkb_fd_jacobian_device(const mkb_device_batch* templates, const mkb_residual
                            double* r0, int64_t* status_changes, void* workspace,
                            size_t workspace_bytes, void* stream);
 
-/* Adjoint sweep with checkpoints every 4 surfaces, then the piston projection: replaces
+/* Adjoint sweep over kept or checkpointed states, then the piston projection: replaces
  * DeviceAdjointJacobian::compute (src/cuda/adjoint_jacobian.cu:401) and
- * adjoint_jacobian_cpu (src/optim/adjoint_jacobian.cpp:370). status [runs][rays]. */
+ * adjoint_jacobian_cpu (src/optim/adjoint_jacobian.cpp:370). status [runs][rays].
+ * The workspace is mkb_adjoint_jacobian_plan_workspace_bytes(templates, plan, runs) bytes, the run
+ * records and the kept states of at most 444 blocks of 128 rays. The size without a plan is
+ * accepted too; it suits the fused adjoint below with any plan and any variables. */
+size_t mkb_adjoint_jacobian_plan_workspace_bytes(const mkb_device_batch* templates,
+                                                 const mkb_residual_plan* plan, int32_t runs);
 size_t mkb_adjoint_jacobian_workspace_bytes(const mkb_device_batch* templates, int32_t runs);
 int mkb_adjoint_jacobian_device(const mkb_device_batch* templates, const mkb_residual_plan* plan,
                                 const mkb_variables* vars, const double* x0, int32_t runs,
@@ -343,8 +348,15 @@ int mkb_adjoint_jacobian_device(const mkb_device_batch* templates, const mkb_res
  * the piston-projected adjoint rows (and the penalty rows), J never written to memory.
  * Replaces DeviceAdjointJacobian::compute + DeviceNormalEquations::compute for the LM. The
  * rows are computed in the plan's precision (FP64: the rows of the exact path; FP64_FMA:
- * contracted), the contraction runs on FP64 tensor cores; the workspace is
- * mkb_adjoint_jacobian_workspace_bytes(templates, runs). */
+ * contracted), the contraction runs on FP64 tensor cores. The workspace is
+ * mkb_adjoint_normal_equations_workspace_bytes(templates, plan, vars, 0, runs) bytes: the run
+ * records, and per block that the call starts (at most one for every 512 rays, whole tuples, of
+ * every run; at most 148, MIXED and FP32_BULK 296) the states of 256 rays. The larger
+ * mkb_adjoint_jacobian_workspace_bytes(templates, runs) suits every plan and every variable set. */
+size_t mkb_adjoint_normal_equations_workspace_bytes(const mkb_device_batch* templates,
+                                                    const mkb_residual_plan* plan,
+                                                    const mkb_variables* vars,
+                                                    int32_t per_run_variables, int32_t runs);
 int mkb_adjoint_normal_equations_device(const mkb_device_batch* templates,
                                         const mkb_residual_plan* plan, const mkb_variables* vars,
                                         const double* x0, int32_t runs, double* gram,
@@ -353,7 +365,9 @@ int mkb_adjoint_normal_equations_device(const mkb_device_batch* templates,
 /* The same for an uneven batch: `vars` is an array of `runs` variable sets (one per run; the
  * counts may differ), x0 rows are strided by the largest count Pmax and gram [runs] slots by
  * (Pmax + 1)^2 (run i's (P_i + 1)^2 matrix dense at the start of its slot). Templates with
- * variant_surfaces must hold one template per run. */
+ * variant_surfaces must hold one template per run. The workspace is
+ * mkb_adjoint_normal_equations_workspace_bytes(templates, plan, vars, 1, runs) bytes; the size
+ * without a plan suits every plan. */
 size_t mkb_adjoint_normal_equations_runs_workspace_bytes(const mkb_device_batch* templates,
                                                          const mkb_variables* vars,
                                                          int32_t runs);

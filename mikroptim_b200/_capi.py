@@ -280,10 +280,14 @@ def _declare(lib: C.CDLL) -> None:
                                            c.c_void_p]
     lib.mkb_adjoint_jacobian_workspace_bytes.restype = c.c_size_t
     lib.mkb_adjoint_jacobian_workspace_bytes.argtypes = [PB, c.c_int32]
+    lib.mkb_adjoint_jacobian_plan_workspace_bytes.restype = c.c_size_t
+    lib.mkb_adjoint_jacobian_plan_workspace_bytes.argtypes = [PB, PP, c.c_int32]
     lib.mkb_adjoint_jacobian_device.restype = c.c_int
     lib.mkb_adjoint_jacobian_device.argtypes = [PB, PP, PV, c.c_void_p, c.c_int32, c.c_void_p,
                                                 c.c_void_p, c.c_void_p, c.c_void_p, c.c_size_t,
                                                 c.c_void_p]
+    lib.mkb_adjoint_normal_equations_workspace_bytes.restype = c.c_size_t
+    lib.mkb_adjoint_normal_equations_workspace_bytes.argtypes = [PB, PP, PV, c.c_int32, c.c_int32]
     lib.mkb_adjoint_normal_equations_device.restype = c.c_int
     lib.mkb_adjoint_normal_equations_device.argtypes = [PB, PP, PV, c.c_void_p, c.c_int32,
                                                         c.c_void_p, c.c_void_p, c.c_size_t,

@@ -79,7 +79,8 @@ class AdjointProblem:
         x = self._x(x)
         runs = x.shape[0]
         b = self.templates.c_struct()
-        need = int(self._lib.mkb_adjoint_jacobian_workspace_bytes(C.byref(b), runs))
+        need = int(self._lib.mkb_adjoint_normal_equations_workspace_bytes(
+            C.byref(b), C.byref(self._plan), C.byref(self._vars), 0, runs))
         ws = torch.empty(max(need, 1), dtype=torch.uint8, device=self.device)
         gram = torch.empty((runs, self.P + 1, self.P + 1), dtype=torch.float64,
                            device=self.device)

@@ -554,8 +554,10 @@ constexpr int kSlotDoubles = 10;
 constexpr bool kFusedDual = true;   // one two-seed sweep for rays with both rows
 constexpr int kMaxTileCols = (MKB_MAX_VARIABLES + 1 + 7) / 8;                    // 9
 constexpr int kMaxTilePairs = kMaxTileCols * (kMaxTileCols + 1) / 2;             // 45
-constexpr int kMaxFusedSlots = 148 * 2;  // persistent CTAs at most (SMs x resident CTAs)
-constexpr int kMaxRowsSlots = 148 * 4;   // of kept_rows_kernel
+// persistent CTAs at most (SMs x resident CTAs): of the fused kernel with FP64 and with FP32 rows,
+// of kept_rows_kernel
+constexpr int kFusedCtas = 148, kFusedCtasFloat = 148 * 2;
+constexpr int kMaxRowsSlots = 148 * kRowsMinBlocks;
 // Pieces of a run: whole tuples, at least kPieceRays rays (more when a run would otherwise have
 // more than kMaxPieces); at most kPieceGroups groups of consecutive pieces. 512 rays are two
 // chunks (about 0.1 ms of one CTA), against some 2 us to stage a record and store a piece's sum.
@@ -1068,6 +1070,8 @@ struct FusedPieces {
     int first[kPieceGroups + 1];     // first piece of every group, then the piece count
 };
 
+int groups_of(int pieces) { return pieces < kPieceGroups ? pieces : kPieceGroups; }
+
 FusedPieces make_pieces(const TraceParams& p) {
     FusedPieces c{};
     int target = kPieceRays;
@@ -1081,18 +1085,18 @@ FusedPieces make_pieces(const TraceParams& p) {
         if (have >= target) have = 0;
     }
     c.ray[c.count] = p.rays;
-    c.groups = c.count < kPieceGroups ? c.count : kPieceGroups;
+    c.groups = groups_of(c.count);
     for (int g = 0; g <= c.groups; ++g) c.first[g] = g * c.count / c.groups;
     return c;
 }
 
 // Items per run, 1, the groups or the pieces: the fewest that give every CTA of the grid
 // kItemsPerCta items (fewer leave the last round of the queue half empty), as long as their
-// sums fit the scratch. 512 objectives of 29 pieces on 444 CTAs of 128 threads: 17.5 ms with one item per run
-// (1.15 rounds of the queue), 11.0 ms with one per piece.
-int choose_items(const FusedPieces& c, int runs, int grid, size_t sum_bytes, size_t room) {
+// sums fit the scratch. 512 objectives of 29 pieces on 444 CTAs of 128 threads: 17.5 ms with one
+// item per run (1.15 rounds of the queue), 11.0 ms with one per piece.
+int choose_items(int pieces, int runs, int grid, size_t sum_bytes, size_t room) {
     int items = 1;
-    for (const int n : {c.groups, c.count}) {
+    for (const int n : {groups_of(pieces), pieces}) {
         if (static_cast<int64_t>(items) * runs >= static_cast<int64_t>(kItemsPerCta) * grid) break;
         if (sum_bytes * static_cast<size_t>(runs) * n > room) break;
         items = n;
@@ -1657,34 +1661,59 @@ size_t tile_pairs(int P) {
     const size_t n = static_cast<size_t>(fused_np(P) / 8);
     return n * (n + 1) / 2;
 }
-int64_t fused_slot_doubles(int P, int S) {
-    return static_cast<int64_t>(fused_np(P) + kSlotDoubles * S) * kFusedThreads +
-           2 * 64 * static_cast<int64_t>(tile_pairs(P));
+// doubles of a CTA's slot: penalty rows and checkpoints (FP32 in MIXED and FP32_BULK), then the
+// group and run sums
+int64_t fused_slot_doubles(int P, int S, bool float_rows) {
+    const int64_t values = static_cast<int64_t>(fused_np(P) + kSlotDoubles * S) * kFusedThreads;
+    return (float_rows ? values / 2 : values) + 2 * 64 * static_cast<int64_t>(tile_pairs(P));
 }
 // The scratch: the queue counter and the runs' item counters, the items' sums, the CTAs' slots
-// (each part 256-byte aligned).
+// (each part 256-byte aligned). It is sized by the plan's pieces: a CTA works on one item, so
+// there are no more slots than items, and a run that is one item leaves no sum.
 struct FusedScratch {
     size_t counters, partial, slots;  // bytes of the first two, number of slots
+    size_t bytes;                     // of all
 };
-FusedScratch fused_scratch(int runs, int P) {
+FusedScratch fused_scratch(int runs, int P, int S, int pieces, bool float_rows) {
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t n = static_cast<size_t>(runs);
+    const size_t sum_bytes = tile_pairs(P) * 64 * sizeof(double);
+    const int ctas = float_rows ? kFusedCtasFloat : kFusedCtas;
+    // the launch's grid is at most `ctas`, and a smaller grid asks for no more items
+    const size_t items = choose_items(pieces, runs, ctas, sum_bytes, kMaxPartialBytes);
     FusedScratch z;
     z.counters = al((n + 64) * sizeof(int));
-    z.partial = n * kMaxPieces * tile_pairs(P) * 64 * sizeof(double);
-    if (z.partial > kMaxPartialBytes) z.partial = kMaxPartialBytes;
-    z.partial = al(z.partial);
-    z.slots = n * kMaxPieces < kMaxFusedSlots ? n * kMaxPieces : kMaxFusedSlots;
+    z.partial = items > 1 ? al(n * items * sum_bytes) : 0;
+    z.slots = n * items < static_cast<size_t>(ctas) ? n * items : ctas;
+    z.bytes = z.counters + z.partial +
+              z.slots * fused_slot_doubles(P, S, float_rows) * sizeof(double);
     return z;
+}
+bool float_rows_of(int precision) {
+    return precision == MKB_PRECISION_MIXED || precision == MKB_PRECISION_FP32_BULK;
 }
 }  // namespace
 
 // Global scratch of the fused kernel: the counters and the items' sums, then one slot per
 // persistent CTA with its penalty rows and its checkpoints (rewritten for every chunk, so it
 // stays in L2) and its group and run sums.
-size_t fused_scratch_bytes(int runs, int P, int S) {
-    const FusedScratch z = fused_scratch(runs, P);
-    return z.counters + z.partial + z.slots * fused_slot_doubles(P, S) * sizeof(double);
+size_t fused_scratch_bytes(const TraceParams& tp, int P, int precision) {
+    return fused_scratch(tp.V, P, tp.S, make_pieces(tp).count, float_rows_of(precision)).bytes;
+}
+
+// The largest over every plan of `tuples` tuples (a piece is whole tuples), every precision and
+// every P up to p_max.
+size_t fused_scratch_bound(int runs, int p_max, int S, int tuples) {
+    size_t most = 0;
+    for (int columns = 1; columns <= fused_np(p_max) / 8; ++columns) {
+        const int P = columns * 8 - 1 < p_max ? columns * 8 - 1 : p_max;
+        for (int pieces = 1; pieces <= tuples && pieces <= kMaxPieces; ++pieces)
+            for (const bool float_rows : {false, true}) {
+                const size_t b = fused_scratch(runs, P, S, pieces, float_rows).bytes;
+                most = b > most ? b : most;
+            }
+    }
+    return most;
 }
 
 int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double* records,
@@ -1698,31 +1727,29 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
     }
     if (tp.V <= 0) return MKB_OK;
     const int p_max = rv.table != nullptr ? rv.stride : vp.P;  // sizes the shared memory
-    if (scratch == nullptr || scratch_bytes < fused_scratch_bytes(tp.V, p_max, tp.S)) {
-        set_error("fused adjoint: scratch of %zu bytes needed",
-                  fused_scratch_bytes(tp.V, p_max, tp.S));
+    const bool float_rows = float_rows_of(precision);
+    FusedArgs fa;
+    fa.pc = make_pieces(tp);
+    const FusedScratch z = fused_scratch(tp.V, p_max, tp.S, fa.pc.count, float_rows);
+    if (scratch == nullptr || scratch_bytes < z.bytes) {
+        set_error("fused adjoint: scratch of %zu bytes needed", z.bytes);
         return MKB_ERR_WORKSPACE;
     }
-    FusedArgs fa;
     fa.ap.t = tp;
     fa.ap.v = vp;
     fa.ap.rows = 0;
     fa.records = records;
     fa.gram = gram;
-    const FusedScratch z = fused_scratch(tp.V, p_max);
     fa.queue = static_cast<int*>(scratch);
     fa.done = fa.queue + 64;
     fa.partial = reinterpret_cast<double*>(static_cast<char*>(scratch) + z.counters);
     fa.scratch = reinterpret_cast<double*>(static_cast<char*>(scratch) + z.counters + z.partial);
-    fa.pc = make_pieces(tp);
-    fa.slot_doubles = fused_slot_doubles(p_max, tp.S);
+    fa.slot_doubles = fused_slot_doubles(p_max, tp.S, float_rows);
     fa.run_mask = run_mask;
     fa.order = order;
     fa.vt = rv.table;
     fa.p_max = p_max;
     fa.gram_stride = static_cast<int64_t>(p_max + 1) * (p_max + 1);
-    const bool float_rows =
-        precision == MKB_PRECISION_MIXED || precision == MKB_PRECISION_FP32_BULK;
     const size_t smem = fused_adjoint_smem(tp, p_max, float_rows ? sizeof(float) : sizeof(double));
     if (precision == MKB_PRECISION_FP32_BULK && (tp.non_coaxial || tp.G > 0)) {
         set_error("fused adjoint: FP32_BULK is built for coaxial batches without ghost plates");
@@ -1795,7 +1822,8 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
     }
     int grid = sms * per_sm;
     if (grid > static_cast<int>(z.slots)) grid = static_cast<int>(z.slots);
-    fa.items = choose_items(fa.pc, tp.V, grid, tile_pairs(p_max) * 64 * sizeof(double), z.partial);
+    fa.items = choose_items(fa.pc.count, tp.V, grid, tile_pairs(p_max) * 64 * sizeof(double),
+                            z.partial);
     if (grid > static_cast<int64_t>(tp.V) * fa.items) grid = tp.V * fa.items;
     err = cudaMemsetAsync(fa.queue, 0, (static_cast<size_t>(tp.V) + 64) * sizeof(int), stream);
     if (err != cudaSuccess) return cuda_status(err, "fused adjoint: clear queue");

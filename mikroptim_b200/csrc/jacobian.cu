@@ -269,6 +269,20 @@ int fd_jacobian(const mkb_device_batch* templates, const mkb_residual_plan* plan
 namespace mkb {
 namespace {
 
+// The workspace of the fused adjoint: the run records, with per-run variables their table, and
+// the kernel's scratch.
+size_t normal_equations_bytes(const TraceParams& tp, int p_max, int precision, bool per_run) {
+    const size_t runs = static_cast<size_t>(tp.V);
+    return align256(sizeof(double) * runs * tp.stride) +
+           (per_run ? align256(sizeof(VarParams) * runs) : 0) +
+           fused_scratch_bytes(tp, p_max, precision);
+}
+// The workspace of the materialised adjoint: the run records and its kernel's scratch.
+size_t jacobian_bytes(const TraceParams& tp) {
+    return align256(sizeof(double) * static_cast<size_t>(tp.V) * tp.stride) +
+           adjoint_rows_scratch_bytes(tp);
+}
+
 // The fused adjoint + normal equations of mkb_adjoint_normal_equations_device and, with
 // per_run, of mkb_adjoint_normal_equations_runs_device (vars: one set per run).
 int adjoint_normal_equations(const mkb_device_batch* templates, const mkb_residual_plan* plan,
@@ -317,9 +331,7 @@ int adjoint_normal_equations(const mkb_device_batch* templates, const mkb_residu
             pmax = table[r].P > pmax ? table[r].P : pmax;
         }
     }
-    const size_t need = per_run ? mkb_adjoint_normal_equations_runs_workspace_bytes(templates,
-                                                                                    vars, runs)
-                                : mkb_adjoint_jacobian_workspace_bytes(templates, runs);
+    const size_t need = normal_equations_bytes(tp, pmax, plan->precision, per_run);
     if (workspace == nullptr || workspace_bytes < need) {
         set_error("adjoint normal equations: workspace of %zu bytes needed", need);
         return MKB_ERR_WORKSPACE;
@@ -423,7 +435,18 @@ int mkb_fd_jacobian_device(const mkb_device_batch* templates, const mkb_residual
 size_t mkb_adjoint_jacobian_workspace_bytes(const mkb_device_batch* templates, int32_t runs) {
     if (templates == nullptr || runs < 0) return 0;
     return align256(sizeof(double) * static_cast<size_t>(runs) * templates->record_stride) +
-           fused_scratch_bytes(runs, MKB_MAX_VARIABLES, templates->surfaces);
+           fused_scratch_bound(runs, MKB_MAX_VARIABLES, templates->surfaces,
+                               templates->fields * templates->wavelengths);
+}
+
+size_t mkb_adjoint_jacobian_plan_workspace_bytes(const mkb_device_batch* templates,
+                                                 const mkb_residual_plan* plan, int32_t runs) {
+    if (templates == nullptr || runs < 0) return 0;
+    TraceParams tp;
+    mkb_device_batch b = *templates;
+    b.variants = runs;
+    if (make_trace_params(&b, plan, pack_rays_default(), &tp) != MKB_OK) return 0;
+    return jacobian_bytes(tp);
 }
 
 int mkb_adjoint_jacobian_device(const mkb_device_batch* templates, const mkb_residual_plan* plan,
@@ -461,8 +484,11 @@ int mkb_adjoint_jacobian_device(const mkb_device_batch* templates, const mkb_res
         set_error("adjoint jacobian: null pointer");
         return MKB_ERR_ARGUMENT;
     }
-    const size_t need = mkb_adjoint_jacobian_workspace_bytes(templates, runs);
-    if (workspace == nullptr || workspace_bytes < need) {
+    // the size without a plan may be below the plan's: fewer CTAs share it
+    const size_t need = jacobian_bytes(tp);
+    if (workspace == nullptr ||
+        (workspace_bytes < need &&
+         workspace_bytes < mkb_adjoint_jacobian_workspace_bytes(templates, runs))) {
         set_error("adjoint jacobian: workspace of %zu bytes needed", need);
         return MKB_ERR_WORKSPACE;
     }
@@ -500,6 +526,22 @@ int mkb_adjoint_normal_equations_device(const mkb_device_batch* templates,
                                     workspace_bytes, static_cast<cudaStream_t>(stream_ptr));
 }
 
+size_t mkb_adjoint_normal_equations_workspace_bytes(const mkb_device_batch* templates,
+                                                    const mkb_residual_plan* plan,
+                                                    const mkb_variables* vars,
+                                                    int32_t per_run_variables, int32_t runs) {
+    if (templates == nullptr || vars == nullptr || runs < 0) return 0;
+    int pmax = 1;
+    for (int r = 0; r < (per_run_variables != 0 ? runs : 1); ++r)
+        pmax = vars[r].count > pmax ? vars[r].count : pmax;
+    if (pmax > MKB_MAX_VARIABLES) return 0;
+    TraceParams tp;
+    mkb_device_batch b = *templates;
+    b.variants = runs;
+    if (make_trace_params(&b, plan, pack_rays_default(), &tp) != MKB_OK) return 0;
+    return normal_equations_bytes(tp, pmax, plan->precision, per_run_variables != 0);
+}
+
 size_t mkb_adjoint_normal_equations_runs_workspace_bytes(const mkb_device_batch* templates,
                                                          const mkb_variables* vars,
                                                          int32_t runs) {
@@ -508,7 +550,8 @@ size_t mkb_adjoint_normal_equations_runs_workspace_bytes(const mkb_device_batch*
     for (int r = 0; r < runs; ++r) pmax = vars[r].count > pmax ? vars[r].count : pmax;
     if (pmax > MKB_MAX_VARIABLES) return 0;
     return align256(sizeof(double) * static_cast<size_t>(runs) * templates->record_stride) +
-           fused_scratch_bytes(runs, pmax, templates->surfaces) +
+           fused_scratch_bound(runs, pmax, templates->surfaces,
+                               templates->fields * templates->wavelengths) +
            align256(sizeof(VarParams) * static_cast<size_t>(runs));
 }
 

@@ -55,7 +55,7 @@ int launch_apply(const VarParams& vp, const RecordLayout& lay, const double* tem
                  int n_templates, const double* x, double* out, int runs, cudaStream_t stream,
                  RunVars rv = {});
 // scratch: adjoint_rows_scratch_bytes(tp) fill the GPU; fewer CTAs run with less (at least one
-// slot of the fused scratch)
+// slot)
 size_t adjoint_rows_scratch_bytes(const TraceParams& tp);
 int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows,
                         const double* records, double* J, bool exact, void* scratch,
@@ -66,7 +66,10 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
                         double* gram, void* scratch, size_t scratch_bytes, int precision,
                         cudaStream_t stream, const int* run_mask = nullptr, RunVars rv = {},
                         const int* order = nullptr);
-size_t fused_scratch_bytes(int runs, int P, int S);
+// scratch of launch_adjoint_gram (P: the largest of the runs), and the largest over every plan of
+// `tuples` tuples, every precision and every P up to p_max
+size_t fused_scratch_bytes(const TraceParams& tp, int P, int precision);
+size_t fused_scratch_bound(int runs, int p_max, int S, int tuples);
 
 // gram.cu
 int launch_gram(const double* J, const double* r, int runs, int P, int64_t R, double* gram,

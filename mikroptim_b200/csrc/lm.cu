@@ -589,7 +589,7 @@ LmLayout lm_layout(char* base, const LmSetup& s, int runs, const mkb_device_batc
     L.trial_merit = reinterpret_cast<double*>(take(8 * r));
     L.trial_failed = reinterpret_cast<int64_t*>(take(8 * r));
     L.trial_hard = reinterpret_cast<int64_t*>(take(8 * r));
-    L.fused_ws_bytes = s.fused ? fused_scratch_bytes(runs, s.pmax, tp.S)
+    L.fused_ws_bytes = s.fused ? fused_scratch_bytes(tp, s.pmax, s.precision)
                        : s.fd  ? 0
                                : adjoint_rows_scratch_bytes(tp);
     L.fused_ws = take(L.fused_ws_bytes);

@@ -1007,7 +1007,7 @@ def adjoint_jacobian_device(templates: DeviceSystemBatch, layout: ResidualLayout
     R = layout.trace_rows
     b = templates.c_struct()
     plan = layout.plan(host)
-    need = int(lib.mkb_adjoint_jacobian_workspace_bytes(C.byref(b), runs))
+    need = int(lib.mkb_adjoint_jacobian_plan_workspace_bytes(C.byref(b), C.byref(plan), runs))
     ws = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
     J = torch.empty((runs, P, R), dtype=torch.float64, device=dev)
     r0 = torch.empty((runs, R), dtype=torch.float64, device=dev)
@@ -1722,10 +1722,11 @@ def adjoint_normal_equations_device(templates: DeviceSystemBatch, layout: Residu
     runs, P = x0.shape
     b = templates.c_struct()
     plan = layout.plan(host)
-    need = int(lib.mkb_adjoint_jacobian_workspace_bytes(C.byref(b), runs))
+    vs = variables.c_struct()
+    need = int(lib.mkb_adjoint_normal_equations_workspace_bytes(C.byref(b), C.byref(plan),
+                                                                C.byref(vs), 0, runs))
     ws = torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
     gram = torch.empty((runs, P + 1, P + 1), dtype=torch.float64, device=dev)
-    vs = variables.c_struct()
     rc = lib.mkb_adjoint_normal_equations_device(C.byref(b), C.byref(plan), C.byref(vs),
                                                  C.c_void_p(x0.data_ptr()), runs,
                                                  C.c_void_p(gram.data_ptr()),
@@ -1799,7 +1800,8 @@ def adjoint_normal_equations_runs_device(templates: DeviceSystemBatch, layout: R
     b = templates.c_struct()
     plan = layout.plan(host)
     pv = rv.pointer
-    need = int(lib.mkb_adjoint_normal_equations_runs_workspace_bytes(C.byref(b), pv, runs))
+    need = int(lib.mkb_adjoint_normal_equations_workspace_bytes(C.byref(b), C.byref(plan), pv, 1,
+                                                                runs))
     ws = workspace if workspace is not None and workspace.numel() >= need else \
         torch.empty(max(need, 1), dtype=torch.uint8, device=dev)
     gram = torch.zeros((runs, pmax + 1, pmax + 1), dtype=torch.float64, device=dev)

@@ -1024,7 +1024,7 @@ void DeviceAdjointJacobian::compute(TraceEngine& engine, const VariableSet& vari
     auto* r0 = static_cast<double*>(r0_.reserve(sizeof(double) * runs * R));
     auto* st = static_cast<uint8_t*>(status_.reserve(static_cast<size_t>(runs) *
                                                      layout.rays_per_variant()));
-    workspace_.reserve(mkb_adjoint_jacobian_workspace_bytes(&t, runs));
+    workspace_.reserve(mkb_adjoint_jacobian_plan_workspace_bytes(&t, plan->get(), runs));
     check(mkb_adjoint_jacobian_device(&t, plan->get(), &v, x, runs, J, r0, st, workspace_.get(),
                                       workspace_.bytes(), engine.stream()),
           "adjoint jacobian");

@@ -60,3 +60,32 @@ def test_rows_and_projection_equal_the_oracle(rings, spokes, glass, failure):
     J = J.cpu().numpy()
     # bit for bit, the signs of zeros included
     assert np.array_equal(J.view(np.int64), Jo.view(np.int64)), np.argwhere(J != Jo)[:5]
+
+
+def test_fewer_blocks_share_the_workspace_sized_without_a_plan():
+    """The size without a plan is below the plan's here: the rows are the same bits, and one byte
+    less is refused."""
+    import ctypes as C
+    from mikroptim_b200 import _capi
+    lib = _capi.lib()
+    b, st, vs, x0 = workloads.sweep(4, surfaces=30, wavelengths=7, rings=16, spokes=32)
+    lay = ResidualLayout(b.topology, st)
+    db = engine.DeviceSystemBatch(b)
+    J, r, s = engine.adjoint_jacobian_device(db, lay, b, vs, x0)
+    t, plan, v = db.c_struct(), lay.plan(b), vs.c_struct()
+    need = int(lib.mkb_adjoint_jacobian_workspace_bytes(C.byref(t), 4))
+    assert need < int(lib.mkb_adjoint_jacobian_plan_workspace_bytes(C.byref(t), C.byref(plan), 4))
+    x = engine._dev_f64(x0, db.device)
+    ws = torch.empty(need, dtype=torch.uint8, device=db.device)
+    J2, r2, s2 = torch.empty_like(J), torch.empty_like(r), torch.empty_like(s)
+
+    def call(nbytes):
+        return lib.mkb_adjoint_jacobian_device(
+            C.byref(t), C.byref(plan), C.byref(v), C.c_void_p(x.data_ptr()), 4,
+            *(C.c_void_p(a.data_ptr()) for a in (J2, r2, s2, ws)), nbytes, None)
+    assert call(need - 1) == _capi.MKB_ERR_WORKSPACE
+    torch.cuda.synchronize()
+    _capi.check(call(need), "adjoint jacobian")
+    torch.cuda.synchronize()
+    assert torch.equal(J2.view(torch.int64), J.view(torch.int64)) and torch.equal(r2, r)
+    assert torch.equal(s2, s)
