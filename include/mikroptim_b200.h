@@ -351,7 +351,8 @@ int mkb_adjoint_jacobian_device(const mkb_device_batch* templates, const mkb_res
  * contracted), the contraction runs on FP64 tensor cores. The workspace is
  * mkb_adjoint_normal_equations_workspace_bytes(templates, plan, vars, 0, runs) bytes: the run
  * records, and per block that the call starts (at most one for every 512 rays, whole tuples, of
- * every run; at most 148, MIXED and FP32_BULK 296) the states of 256 rays. The larger
+ * every run; at most 148, MIXED and FP32_BULK 296) the states of 256 rays -- in plans of at most
+ * 3,072 rays, one for every 256, at most 444 and 592, of 128 rays. The larger
  * mkb_adjoint_jacobian_workspace_bytes(templates, runs) suits every plan and every variable set. */
 size_t mkb_adjoint_normal_equations_workspace_bytes(const mkb_device_batch* templates,
                                                     const mkb_residual_plan* plan,

@@ -502,8 +502,8 @@ MKB_DEFINE_ERROR_READER(adjoint_device_error)
 
 namespace mkb {
 // ---- fused adjoint + normal equations ---------------------------------------------------------
-// Persistent CTAs take runs off a work queue; a CTA streams the run's rays in chunks of
-// kFusedThreads (one ray per thread):
+// Persistent CTAs take runs off a work queue; a CTA streams the run's rays in chunks of one ray
+// per thread:
 //   A  forward trace that stores the ray state entering every surface in the CTA's slot of an
 //      L2-resident global scratch (thread-minor, coalesced), then ONE reverse sweep over those
 //      states carrying two adjoint vectors (seed OPL = 1 and seed penalty = 1) that share the
@@ -524,8 +524,8 @@ namespace mkb {
 //      s_p sqrt(W) p_k) are loaded from the scratch slot into Y and accumulated the same way.
 // Output: gram [runs][P+1][P+1] as the normal-equation kernels write it.
 //
-// A run is cut into pieces of whole tuples (FusedPieces: about kPieceRays rays each) and the
-// pieces into at most kPieceGroups groups, from the plan alone. A piece accumulates from zero,
+// A run is cut into pieces of whole tuples (make_pieces) and the pieces into at most
+// kPieceGroups groups, from the plan alone. A piece accumulates from zero,
 // a group is the sum of its pieces and a run the sum of its groups, each in ascending order,
 // whoever computes them: one CTA takes a whole run, a group or a piece off the queue
 // (choose_items), so a run's bits do not depend on the batch it is in. With more than one item
@@ -533,20 +533,28 @@ namespace mkb {
 // counter per run, no CTA waits) adds them up.
 namespace {
 
-// One CTA of 256 threads (FP64: up to 255 registers, no spills) or two (MIXED, FP32_BULK: 128
-// registers) per SM. Against CTAs of 128 threads, three or four to an SM, the warps of a
-// scheduler are in the same phase more often and share its instruction fetches (ncu: a quarter
-// of the stalls of 128-thread CTAs were missing instructions), one accumulator and record serve
-// twice the rays, and the FP64 instances no longer spill. 128 -> 256 threads: 512 objectives
-// (FP64) 9.62 -> 9.33 ms, 2,048 uneven systems (MIXED) 21.9 -> 19.9 ms, merit and gradient of
-// 1,024 toleranced samples 17.8 -> 17.0 ms, six LM iterations of 512 uneven systems (FP64_FMA)
-// 53.5 -> 50.2 ms. 384 threads of 168 registers: 10.8 ms where 128 threads took 11.0 (FP64),
-// 24.2 where they took 21.9 (MIXED).
-constexpr int kFusedThreads = 256;
-constexpr int kFusedWarps = kFusedThreads / 32;
+// One CTA of 256 threads (FP64: 242 to 255 registers, nothing spilled without plates, transforms,
+// glass and stop, else at most 136 bytes of stores) or two (MIXED, FP32_BULK: 128 registers) per SM;
+// in plans of few rays (fused_threads) CTAs of 128 threads, three (FP64: 168 registers) or four. In
+// larger CTAs the warps of a scheduler are in the same phase more often and share its instruction
+// fetches (ncu: a quarter of the stalls of 128-thread CTAs were missing instructions), and one
+// accumulator and record serve twice the rays. 128 -> 256 threads: 512 objectives (FP64) 9.62 ->
+// 9.33 ms, 2,048 uneven systems (MIXED) 21.9 -> 19.9 ms, merit and gradient of 1,024 toleranced
+// samples 17.8 -> 17.0 ms, six LM iterations of 512 uneven systems (FP64_FMA) 53.5 -> 50.2 ms. 384
+// threads of 168 registers: 10.8 ms where 128 threads took 11.0 (FP64), 24.2 where they took 21.9
+// (MIXED).
+// Two MIXED CTAs fit an SM's shared memory up to 63 variables (64 surfaces of 7 wavelengths too); at
+// 64 from 20 surfaces of 7 wavelengths on it is one: 1,024 uneven systems with a widest run of 63
+// variables 11.2 ms, of 64 15.9 ms.
+constexpr int kFusedThreads = 256, kFusedThreadsSmall = 128;
+constexpr int kSmallPlanRays = 3072;  // most rays of a run that takes the small block
+// CTAs per SM that the registers are budgeted for
+constexpr int fused_ctas_per_sm(int threads, bool float_rows) {
+    return threads == kFusedThreads ? (float_rows ? 2 : 1) : (float_rows ? 4 : 3);
+}
 constexpr int kRowsThreads = 128;   // of kept_rows_kernel: three CTAs of 168 registers per SM
 constexpr int kRowsMinBlocks = 3;   // (640 us; 256 threads took 800 us)
-constexpr int kExtraRows = 8;
+constexpr int kExtraStride = 4;  // a chunk's extra row, padded to the four rows of a DMMA step
 // Per ray and table surface c the forward pass keeps, in the CTA's scratch slot, the state
 // entering the step c -> c + 1 and that step's StepLocal quantities but mu (kSlotDoubles
 // values; mu = n / n' per surface and wavelength is in a shared-memory table of the run).
@@ -556,12 +564,11 @@ constexpr int kMaxTileCols = (MKB_MAX_VARIABLES + 1 + 7) / 8;                   
 constexpr int kMaxTilePairs = kMaxTileCols * (kMaxTileCols + 1) / 2;             // 45
 // persistent CTAs at most (SMs x resident CTAs): of the fused kernel with FP64 and with FP32 rows,
 // of kept_rows_kernel
-constexpr int kFusedCtas = 148, kFusedCtasFloat = 148 * 2;
+constexpr int kFusedSms = 148;
 constexpr int kMaxRowsSlots = 148 * kRowsMinBlocks;
-// Pieces of a run: whole tuples, at least kPieceRays rays (more when a run would otherwise have
-// more than kMaxPieces); at most kPieceGroups groups of consecutive pieces. 512 rays are two
-// chunks (about 0.1 ms of one CTA), against some 2 us to stage a record and store a piece's sum.
-constexpr int kPieceRays = 512;
+// Pieces of a run (make_pieces): two to four blocks of rays each, at most kPieceGroups groups of
+// consecutive pieces. Two blocks of 256 rays are about 0.1 ms of one CTA, against some 2 us to
+// stage a record and store a piece's sum.
 constexpr int kMaxPieces = 64;
 constexpr int kPieceGroups = 4;
 // Items per CTA of the grid that the split aims at, and the most scratch the items' sums take
@@ -579,10 +586,11 @@ __device__ __forceinline__ int tuple_of(const TraceParams& p, int q) {
     return f * p.L + (q - p.field_offset[f]) / p.sample_count[f];
 }
 
+template <int kT>
 struct FusedShared {
     uint64_t bar;
     SharedTables tab;
-    double w[kFusedThreads];      // sample weight if the ray is in the piston, else 0
+    double w[kT];                 // sample weight if the ray is in the piston, else 0
     int any_pen;                  // chunk has a penalty row (soft mode)
     int item;                     // item taken off the queue
     int last;                     // this CTA brought the last sum of the run
@@ -596,14 +604,15 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 }
 
 // acc += X^T X for X stored column-major, X(k, c) = xt[c * ld + k], k < n (n a multiple of 4;
-// the caller pads with zero rows). Warp w owns tile pairs w, w + 4, ...; the 8 x 8 accumulator
-// tiles live in shared memory in fragment order (acc[pair][lane][2]), loaded and stored around
-// the k loop.
+// the caller pads with zero rows). Warp w owns tile pairs w, w + kT / 32, ...; the 8 x 8
+// accumulator tiles live in shared memory in fragment order (acc[pair][lane][2]), loaded and
+// stored around the k loop.
+template <int kT>
 __device__ __forceinline__ void accumulate(const double* xt, int ld, int n, int pairs,
                                            const int2* tiles, double* acc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
-    for (int e = warp; e < pairs; e += kFusedWarps) {
+    for (int e = warp; e < pairs; e += kT / 32) {
         const double* ca = xt + (tiles[e].x * 8 + gid) * ld + tig;
         const double* cb = xt + (tiles[e].y * 8 + gid) * ld + tig;
         double* a = acc + (e * 32 + lane) * 2;
@@ -617,13 +626,13 @@ __device__ __forceinline__ void accumulate(const double* xt, int ld, int n, int 
 // acc += X^T X for the chunk's rows: X(k, c) = Y[c * ld + k] for the derivative columns
 // (type YT) and R[k] for the residual column c = P (FP64 in every variant), k < n (n a
 // multiple of 4). Fragment columns past P read the zero padding of Y.
-template <class YT>
+template <int kT, class YT>
 __device__ __forceinline__ void accumulate_rows(const YT* Y, const double* R, int ld, int P, int n,
                                                 int pairs, const int2* tiles, double* acc) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;
     const int last = P >> 3;  // the column tile holding the residual column
-    for (int e = warp; e < pairs; e += kFusedWarps) {
+    for (int e = warp; e < pairs; e += kT / 32) {
         const int col_a = tiles[e].x * 8 + gid, col_b = tiles[e].y * 8 + gid;
         const YT* ya = Y + col_a * ld + tig;
         const YT* yb = Y + col_b * ld + tig;
@@ -741,7 +750,7 @@ __device__ void fused_forward(const TraceParams& p, const double* rec, const dou
 
 // fused_forward in MKB_PRECISION_FP32_BULK (coaxial, no ghost plates): the same kept states and
 // step quantities (float slots), traced with step_surface_bulk.
-template <class Q>
+template <class Q, int kT>
 __device__ void fused_forward_bulk(const TraceParams& p, const double* rec, const double* mu_tab,
                                    const RecordLayout& lay, int S, int f, int l,
                                    const Sample& smp, bool soft_mode, Q* ck, int stride_ck,
@@ -773,11 +782,11 @@ __device__ void fused_forward_bulk(const TraceParams& p, const double* rec, cons
     double n_before = idx[l];
     auto keep_state = [&](Q* q) {
         q[0] = Q(r.px);
-        q[1 * kFusedThreads] = Q(r.py);
-        q[2 * kFusedThreads] = Q(r.pz);
-        q[3 * kFusedThreads] = Q(r.dx);
-        q[4 * kFusedThreads] = Q(r.dy);
-        q[5 * kFusedThreads] = Q(r.dz);
+        q[1 * kT] = Q(r.py);
+        q[2 * kT] = Q(r.pz);
+        q[3 * kT] = Q(r.dx);
+        q[4 * kT] = Q(r.dy);
+        q[5 * kT] = Q(r.dz);
     };
     for (int s = 1; s < S; ++s) {
         const double c = p.type[s] == MKB_SURFACE_SPHERE ? curv[s] : 0.0;
@@ -788,10 +797,10 @@ __device__ void fused_forward_bulk(const TraceParams& p, const double* rec, cons
         status = step_surface_bulk<true>(r, thick[s - 1], c, n_before,
                                          static_cast<float>(mu_tab[s * L + l]), sp, branch, &loc);
         if (status != kOk) break;
-        q[6 * kFusedThreads] = Q(loc.s0);
-        q[7 * kFusedThreads] = Q(loc.s);
-        q[8 * kFusedThreads] = Q(loc.root_d);
-        q[9 * kFusedThreads] = Q(loc.root_k);
+        q[6 * kT] = Q(loc.s0);
+        q[7 * kT] = Q(loc.s);
+        q[8 * kT] = Q(loc.root_d);
+        q[9 * kT] = Q(loc.root_k);
         count = s + 1;
         if (s < 32) br_lo |= static_cast<uint64_t>(branch) << (2 * s);
         else br_hi |= static_cast<uint64_t>(branch) << (2 * (s - 32));
@@ -1072,17 +1081,51 @@ struct FusedPieces {
 
 int groups_of(int pieces) { return pieces < kPieceGroups ? pieces : kPieceGroups; }
 
+// Threads of a CTA by the rays of a run. A run's bits depend on it (its rows are summed a block at
+// a time), so nothing of the batch may enter. Plans of few rays leave much of a block of 256 idle
+// and, one CTA to an SM, nothing beside its barriers and staging. With every SM full, 256 -> 128
+// threads (FP64 / MIXED, us): 16,384 singlets of 450 rays 2,240 -> 1,540 / 1,270 -> 1,110, 2,048
+// systems of 648 rays 900 -> 620 / 520 -> 420, 16,384 of 15 rays 1,780 -> 690 / 880 -> 480, 2,048
+// systems of 20 surfaces and 2,520 rays 6,150 -> 4,740 / 3,420 -> 2,970. From 3,640 rays on glass
+// variables (2,840 -> 3,100 / 1,500 -> 1,630) and tilted systems of 21 surfaces lose by it. Below,
+// the widest runs do: 4,096 of P = 61 and 150 rays 2,220 -> 2,640 / 1,270 -> 1,520, where one CTA of
+// two waves stands for two.
+int fused_threads(const TraceParams& p) {
+    return p.rays <= kSmallPlanRays ? kFusedThreadsSmall : kFusedThreads;
+}
+
+// Pieces of whole tuples and of at least two blocks of rays, more when a run would otherwise have
+// more than kMaxPieces. In plans of few rays a block left mostly idle is a large part of the run:
+// there no piece is shorter, and of the ends up to four blocks the first is taken that leaves at
+// most 1/16 of its blocks' threads idle, else the one that leaves the fewest (4,096 systems of
+// 15 tuples of 48 rays, FP64: 2,230 us with the first end, 2,010 us so).
 FusedPieces make_pieces(const TraceParams& p) {
     FusedPieces c{};
-    int target = kPieceRays;
-    if (target < (p.rays + kMaxPieces - 1) / kMaxPieces)
-        target = (p.rays + kMaxPieces - 1) / kMaxPieces;
-    int have = 0;
-    for (int t = 0; t < p.n_tuples; ++t) {
-        const int f = t / p.L;
-        if (have == 0) c.ray[c.count++] = p.field_offset[f] + (t - f * p.L) * p.sample_count[f];
-        have += p.sample_count[f];
-        if (have >= target) have = 0;
+    const int block = fused_threads(p), least = (p.rays + kMaxPieces - 1) / kMaxPieces;
+    const int low = 2 * block > least ? 2 * block : least;
+    const bool first = block == kFusedThreads;
+    int t = 0, ray = 0;
+    while (t < p.n_tuples) {
+        c.ray[c.count++] = ray;
+        int end = p.n_tuples, rays = p.rays - ray, have = 0;
+        double idle = 1.0;  // idle share of the best end so far
+        for (int e = t; e < p.n_tuples && idle > 1.0 / 16.0; ++e) {
+            have += p.sample_count[e / p.L];
+            if (have < low) continue;
+            if (!first &&
+                (p.rays - ray - have < low || (have >= 2 * low && idle < 1.0)))
+                break;
+            const int blocks = (have + block - 1) / block;
+            const double share = 1.0 - static_cast<double>(have) / (blocks * block);
+            if (share < idle) {
+                idle = share;
+                end = e + 1;
+                rays = have;
+            }
+            if (first) break;
+        }
+        t = end;
+        ray += rays;
     }
     c.ray[c.count] = p.rays;
     c.groups = groups_of(c.count);
@@ -1122,31 +1165,28 @@ struct FusedArgs {
     int64_t gram_stride;   // doubles per run of `gram`
 };
 
-template <class N, int kFeat>
-__global__ void __launch_bounds__(kFusedThreads, std::is_same<N, MixedPrecision>::value ||
-                                                         std::is_same<N, BulkPrecision>::value
-                                                     ? 2
-                                                     : 1)
+template <class N, int kFeat, int kT>
+__global__ void __launch_bounds__(
+    kT, fused_ctas_per_sm(kT, std::is_same<typename FusedTypes<N>::Row, float>::value))
 adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
     const TraceParams& p = fa.ap.t;
-    __shared__ FusedShared sh;
+    __shared__ FusedShared<kT> sh;
     __shared__ double aim_sens[(kFeat & 8) != 0 ? 2 * MKB_MAX_VARIABLES : 1];
     extern __shared__ __align__(16) double dyn[];
     const int NPM = fused_np(fa.p_max);  // shared-memory and scratch layout: the largest P
     const int pairs_max = (NPM / 8) * (NPM / 8 + 1) / 2;
-    const int stride_ck = kSlotDoubles * kFusedThreads;
+    const int stride_ck = kSlotDoubles * kT;
     // Column strides = 4 (mod 16) doubles, 4 (mod 32) floats: the lanes of a (half-)warp
     // reading a DMMA fragment (8 columns x 4 rows) then hit different banks; lanes that own
     // consecutive rows of one column (the sweep's writes, the centring) stay conflict-free.
-    constexpr int TS = kFusedThreads + 4;              // column stride of Y
-    constexpr int ES = kExtraRows + 4;                 // column stride of E
+    constexpr int TS = kT + 4;                         // column stride of Y
     double* record = dyn;                              // [stride] (bulk-copy target, 16 B aligned)
     double* mu_tab = record + ((p.stride + 1) & ~1);   // [S + 1][L]: mu of step s - 1 -> s
     using YT = typename FusedTypes<N>::Row;
     YT* Y = reinterpret_cast<YT*>(mu_tab + (((p.S + 1) * p.L + 1) & ~1));  // [NPM][TS]
     double* R = reinterpret_cast<double*>(Y + NPM * TS);  // [TS] the residual column
-    double* E = R + TS;                                // column-major [NPM][ES]
-    double* mu_open = E + NPM * ES;                    // [NPM] running mean of the open tuple
+    double* E = R + TS;                                // column-major [NPM][kExtraStride]
+    double* mu_open = E + NPM * kExtraStride;                    // [NPM] running mean of the open tuple
     double* seg_mean = mu_open + NPM;                  // [kSegBatch][NPM] segment means
     double* seg_w = seg_mean + kSegBatch * NPM;        // [kSegBatch] segment weights
     double* acc = seg_w + kSegBatch;                   // [pairs][32][2] DMMA accumulators
@@ -1157,10 +1197,10 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
     using Keep = typename FusedTypes<N>::Keep;
     YT* pen_slot =
         reinterpret_cast<YT*>(fa.scratch + static_cast<int64_t>(blockIdx.x) * fa.slot_doubles);
-    Keep* ckpt = reinterpret_cast<Keep*>(pen_slot + NPM * kFusedThreads);
+    Keep* ckpt = reinterpret_cast<Keep*>(pen_slot + NPM * kT);
     copy_tables(p, sh.tab);
     // upper-triangle tile pairs in column order: the pairs of a smaller P are a prefix
-    for (int e = tid; e < pairs_max; e += kFusedThreads) {
+    for (int e = tid; e < pairs_max; e += kT) {
         int j = 0, rem = e;
         while (rem >= j + 1) {
             rem -= j + 1;
@@ -1197,13 +1237,13 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
         const int ncols = NP / 8;
         const int pairs = ncols * (ncols + 1) / 2;
         const int S = surfaces_of(p, run);
-        for (int i = tid; i < NPM * ES; i += kFusedThreads) E[i] = 0.0;  // padding stays 0
+        for (int i = tid; i < NPM * kExtraStride; i += kT) E[i] = 0.0;  // padding: 0
         if (!stage_to_shared(record, fa.records + static_cast<int64_t>(run) * p.stride,
                              static_cast<uint32_t>(p.stride * sizeof(double)), &sh.bar, uses++))
             return;
         // mu = n_before / n_after of every step and wavelength, divided as the step divides
         // it (rows 0 and S .. p.S stay 0: no step)
-        for (int i = tid; i < (p.S + 1) * p.L; i += kFusedThreads) {
+        for (int i = tid; i < (p.S + 1) * p.L; i += kT) {
             const int s = i / p.L, l = i - s * p.L;
             using F = typename FusedTypes<N>::Fwd;
             mu_tab[i] = s >= 1 && s < S
@@ -1212,16 +1252,17 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                             : 0.0;
         }
         if constexpr ((kFeat & 8) != 0)  // interior stop: d(a, t0)/dx of the aimed pupil
-            for (int k = tid; k < P; k += kFusedThreads)
+            for (int k = tid; k < P; k += kT)
                 aim_sensitivity(record, lay, v, k, aim_sens[k], aim_sens[MKB_MAX_VARIABLES + k]);
         __syncthreads();
         for (int piece = piece0; piece < piece1; ++piece) {
         const int piece_end = fa.pc.ray[piece + 1];
-        // the open tuple (kept identically by every thread): its index, weight, extra rows
-        int open_tuple = -1, extra = 0;
+        // the open tuple (kept identically by every thread): its index and weight
+        int open_tuple = -1;
+        bool extra = false;  // the chunk has an extra row
         double open_w = 0.0;
-        for (int i = tid; i < pairs * 64; i += kFusedThreads) acc[i] = 0.0;
-        for (int base = fa.pc.ray[piece]; base < piece_end; base += kFusedThreads) {
+        for (int i = tid; i < pairs * 64; i += kT) acc[i] = 0.0;
+        for (int base = fa.pc.ray[piece]; base < piece_end; base += kT) {
             const int q = base + tid;
             YT* row = Y + tid;  // this ray's row, column c at row[c * TS]
             for (int c = 0; c < NP; ++c) row[c * TS] = YT(0);
@@ -1242,11 +1283,11 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                 uint64_t br_lo = 0, br_hi = 0;
                 double opl = 0.0, penalty = 0.0;
                 if constexpr (std::is_same<N, BulkPrecision>::value)
-                    fused_forward_bulk<Keep>(p, record, mu_tab, lay, S, f, l, smp, soft_mode,
+                    fused_forward_bulk<Keep, kT>(p, record, mu_tab, lay, S, f, l, smp, soft_mode,
                                              my_ck, stride_ck, br_lo, br_hi, count,
                                              image_branch, status, soft_first, opl, penalty);
                 else
-                    fused_forward<typename FusedTypes<N>::Fwd, Keep, kFeat, kFusedThreads>(
+                    fused_forward<typename FusedTypes<N>::Fwd, Keep, kFeat, kT>(
                         p, record, mu_tab, lay, S, f, l, smp, soft_mode, my_ck, stride_ck, br_lo,
                         br_hi, count, image_branch, status, soft_first, opl, penalty);
                 const bool piston = in_piston(status);
@@ -1254,7 +1295,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                 const bool pen_sweep = has_pen && soft_first != kOk;
                 const double pfac = has_pen ? p.pscale[tu] * smp.root_weight : 0.0;
                 if (has_pen) {
-                    for (int c = 0; c < NP; ++c) prow[c * kFusedThreads] = YT(0);
+                    for (int c = 0; c < NP; ++c) prow[c * kT] = YT(0);
                     pen_val = pfac * (is_soft(status) ? penalty : penalty + 1.0);
                 }
                 if (piston) opl_val = opl;
@@ -1263,8 +1304,8 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                     if (piston || pen_sweep) {
                         const double so[2] = {piston ? 1.0 : 0.0, 0.0};
                         const double sp[2] = {0.0, pen_sweep ? 1.0 : 0.0};
-                        const RowSinks<2, YT> sinks{{1.0, pfac}, {row, prow}, {TS, kFusedThreads}};
-                        run_backward<N, 2, kFeat, kFusedThreads, ReciprocalDivisor>(
+                        const RowSinks<2, YT> sinks{{1.0, pfac}, {row, prow}, {TS, kT}};
+                        run_backward<N, 2, kFeat, kT, ReciprocalDivisor>(
                             p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
                             count, image_branch, piston, soft_mode, so, sp, sinks, aim_sens);
                     }
@@ -1273,20 +1314,20 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                         const double so[1] = {piston ? 1.0 : 0.0};
                         const double sp[1] = {pen_sweep ? 1.0 : 0.0};
                         const RowSinks<1, YT> sinks{{piston ? 1.0 : pfac}, {piston ? row : prow},
-                                                {piston ? TS : kFusedThreads}};
-                        run_backward<N, 1, kFeat, kFusedThreads, ReciprocalDivisor>(
+                                                {piston ? TS : kT}};
+                        run_backward<N, 1, kFeat, kT, ReciprocalDivisor>(
                             p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
                             count, image_branch, piston, soft_mode, so, sp, sinks, aim_sens);
                     }
                 } else {  // both rows, one sweep each
                     const double so0[1] = {1.0}, sp0[1] = {0.0};
                     const RowSinks<1, YT> s0{{1.0}, {row}, {TS}};
-                    run_backward<N, 1, kFeat, kFusedThreads, ReciprocalDivisor>(
+                    run_backward<N, 1, kFeat, kT, ReciprocalDivisor>(
                             p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
                             count, image_branch, true, soft_mode, so0, sp0, s0, aim_sens);
                     const double so1[1] = {0.0}, sp1[1] = {1.0};
-                    const RowSinks<1, YT> s1{{pfac}, {prow}, {kFusedThreads}};
-                    run_backward<N, 1, kFeat, kFusedThreads, ReciprocalDivisor>(
+                    const RowSinks<1, YT> s1{{pfac}, {prow}, {kT}};
+                    run_backward<N, 1, kFeat, kT, ReciprocalDivisor>(
                             p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
                             count, image_branch, true, soft_mode, so1, sp1, s1, aim_sens);
                 }
@@ -1299,8 +1340,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
             __syncthreads();
             if (has_pen) sh.any_pen = 1;
             // ---- B: centre every tuple segment of the chunk ----
-            const int rows_here = piece_end - base < kFusedThreads ? piece_end - base
-                                                                   : kFusedThreads;
+            const int rows_here = piece_end - base < kT ? piece_end - base : kT;
             // Segments are the chunk's pieces of its tuples; rays are ordered by tuple (f-major,
             // then l), so segment k is tuple t0 + k and its rows follow from the plan alone.
             const int t0 = tuple_of(p, base);
@@ -1326,7 +1366,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                     const int h = lane & 7;
                     const unsigned octet = 0xFFu << (lane & ~7);
                     const int halves = (P >> 1) + 1;  // column pairs of 0 .. P
-                    for (int pr = tid >> 3; pr < kn * halves; pr += kFusedThreads / 8) {
+                    for (int pr = tid >> 3; pr < kn * halves; pr += kT / 8) {
                         const int k = pr / halves, c0 = 2 * (pr - k * halves);
                         const int c1 = c0 < P ? c0 + 1 : P;
                         int a, n;
@@ -1371,7 +1411,8 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                     R[tid] = f != 0.0 ? f * (R[tid] - m[P]) : 0.0;
                 }
                 // B4: the segments merged into the open tuple in row order (threads = columns
-                // for the vectors; the scalar state is updated identically by every thread)
+                // for the vectors; the scalar state is updated identically by every thread).
+                // Only the chunk's first segment can go on with an open tuple: one extra row.
                 for (int k = 0; k < kn; ++k) {
                     const double ws = seg_w[k];
                     if (!(ws > 0.0)) continue;
@@ -1381,43 +1422,33 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                         const double mean = seg_mean[k * NP + tid];
                         if (open) {
                             const double fac = p.scale[t] * sqrt(open_w * ws / (open_w + ws));
-                            E[tid * ES + extra] = fac * (mean - mu_open[tid]);
+                            E[tid * kExtraStride] = fac * (mean - mu_open[tid]);
                             mu_open[tid] += (ws / (open_w + ws)) * (mean - mu_open[tid]);
                         } else {
                             mu_open[tid] = mean;
                         }
                     }
                     if (open) {
-                        extra += 1;
+                        extra = true;
                         open_w += ws;
                     } else {
                         open_tuple = t;
                         open_w = ws;
                     }
-                    if (extra == kExtraRows) {  // flush the extra rows
-                        __syncthreads();
-                        accumulate(E, ES, kExtraRows, pairs, sh.tiles, acc);
-                        __syncthreads();
-                        extra = 0;
-                    }
                 }
-                // zero padding of the pending extra rows to a multiple of 4 (each column by
-                // the thread that writes it)
-                if (tid <= P)
-                    for (int r = extra; r < ((extra + 3) & ~3); ++r) E[tid * ES + r] = 0.0;
                 __syncthreads();
             }
-            // ---- C: the centred rows and the pending extra rows ----
-            accumulate_rows(Y, R, TS, P, (rows_here + 3) & ~3, pairs, sh.tiles, acc);
-            if (extra > 0) accumulate(E, ES, (extra + 3) & ~3, pairs, sh.tiles, acc);
+            // ---- C: the centred rows and the extra row ----
+            accumulate_rows<kT>(Y, R, TS, P, (rows_here + 3) & ~3, pairs, sh.tiles, acc);
+            if (extra) accumulate<kT>(E, kExtraStride, 4, pairs, sh.tiles, acc);
             __syncthreads();
-            extra = 0;
+            extra = false;
             // ---- D: penalty rows ----
             if (sh.any_pen) {
-                for (int c = 0; c < NP; ++c) row[c * TS] = has_pen ? prow[c * kFusedThreads] : YT(0);
+                for (int c = 0; c < NP; ++c) row[c * TS] = has_pen ? prow[c * kT] : YT(0);
                 R[tid] = pen_val;
                 __syncthreads();
-                accumulate_rows(Y, R, TS, P, (rows_here + 3) & ~3, pairs, sh.tiles, acc);
+                accumulate_rows<kT>(Y, R, TS, P, (rows_here + 3) & ~3, pairs, sh.tiles, acc);
                 __syncthreads();
             }
         }
@@ -1427,7 +1458,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
         int g = 0;
         while (piece >= fa.pc.first[g + 1]) ++g;
         const bool opens = piece == fa.pc.first[g], closes = piece + 1 == fa.pc.first[g + 1];
-        for (int i = tid; i < pairs * 64; i += kFusedThreads) {
+        for (int i = tid; i < pairs * 64; i += kT) {
             double s = acc[i];
             if (!opens) s = group_sum[i] + s;
             if (!closes) {
@@ -1442,7 +1473,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
         if (fa.items > 1) {
             // leave the item's sum; the CTA that brings the run's last adds them up
             double* sums = fa.partial + static_cast<int64_t>(run) * fa.items * sum_size;
-            for (int i = tid; i < pairs * 64; i += kFusedThreads)
+            for (int i = tid; i < pairs * 64; i += kT)
                 sums[static_cast<int64_t>(item) * sum_size + i] = acc[i];
             __threadfence();
             __syncthreads();
@@ -1451,7 +1482,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
             if (!sh.last) continue;
             __threadfence();
             const int per = fa.items == fa.pc.groups ? 0 : 1;  // 1: an item is one piece
-            for (int i = tid; i < pairs * 64; i += kFusedThreads) {
+            for (int i = tid; i < pairs * 64; i += kT) {
                 double total = 0.0;
                 for (int g = 0; g < fa.pc.groups; ++g) {
                     const int first = per ? fa.pc.first[g] : g;
@@ -1467,7 +1498,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
         // ---- write the (P+1) x (P+1) symmetric gram ----
         const int n = P + 1;
         double* G = fa.gram + static_cast<int64_t>(run) * fa.gram_stride;
-        for (int i = tid; i < pairs * 64; i += kFusedThreads) {
+        for (int i = tid; i < pairs * 64; i += kT) {
             const int e = i / 64, ln = (i / 2) & 31, h = i & 1;
             const int r = sh.tiles[e].x * 8 + (ln >> 2);
             const int c = sh.tiles[e].y * 8 + 2 * (ln & 3) + h;
@@ -1644,15 +1675,15 @@ int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows
     return cuda_status(cudaGetLastError(), "adjoint rows launch");
 }
 
-size_t fused_adjoint_smem(const TraceParams& tp, int P, size_t row_bytes) {
+size_t fused_adjoint_smem(const TraceParams& tp, int P, size_t row_bytes, int threads) {
     const int NP = fused_np(P);
     const int ncols = NP / 8;
     const int pairs = ncols * (ncols + 1) / 2;
-    const size_t rows = (static_cast<size_t>(kFusedThreads + 4) * NP * row_bytes + 7) / 8;
+    const size_t rows = (static_cast<size_t>(threads + 4) * NP * row_bytes + 7) / 8;
     return sizeof(double) * (static_cast<size_t>((tp.stride + 1) & ~1) +
                              static_cast<size_t>(((tp.S + 1) * tp.L + 1) & ~1) + rows +
-                             (kFusedThreads + 4) +
-                             (kExtraRows + 4) * NP + NP + kSegBatch * (NP + 1) +
+                             (threads + 4) +
+                             kExtraStride * NP + NP + kSegBatch * (NP + 1) +
                              static_cast<size_t>(pairs) * 64);
 }
 
@@ -1663,8 +1694,8 @@ size_t tile_pairs(int P) {
 }
 // doubles of a CTA's slot: penalty rows and checkpoints (FP32 in MIXED and FP32_BULK), then the
 // group and run sums
-int64_t fused_slot_doubles(int P, int S, bool float_rows) {
-    const int64_t values = static_cast<int64_t>(fused_np(P) + kSlotDoubles * S) * kFusedThreads;
+int64_t fused_slot_doubles(int P, int S, bool float_rows, int threads) {
+    const int64_t values = static_cast<int64_t>(fused_np(P) + kSlotDoubles * S) * threads;
     return (float_rows ? values / 2 : values) + 2 * 64 * static_cast<int64_t>(tile_pairs(P));
 }
 // The scratch: the queue counter and the runs' item counters, the items' sums, the CTAs' slots
@@ -1674,11 +1705,11 @@ struct FusedScratch {
     size_t counters, partial, slots;  // bytes of the first two, number of slots
     size_t bytes;                     // of all
 };
-FusedScratch fused_scratch(int runs, int P, int S, int pieces, bool float_rows) {
+FusedScratch fused_scratch(int runs, int P, int S, int pieces, bool float_rows, int threads) {
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t n = static_cast<size_t>(runs);
     const size_t sum_bytes = tile_pairs(P) * 64 * sizeof(double);
-    const int ctas = float_rows ? kFusedCtasFloat : kFusedCtas;
+    const int ctas = kFusedSms * fused_ctas_per_sm(threads, float_rows);
     // the launch's grid is at most `ctas`, and a smaller grid asks for no more items
     const size_t items = choose_items(pieces, runs, ctas, sum_bytes, kMaxPartialBytes);
     FusedScratch z;
@@ -1686,7 +1717,7 @@ FusedScratch fused_scratch(int runs, int P, int S, int pieces, bool float_rows) 
     z.partial = items > 1 ? al(n * items * sum_bytes) : 0;
     z.slots = n * items < static_cast<size_t>(ctas) ? n * items : ctas;
     z.bytes = z.counters + z.partial +
-              z.slots * fused_slot_doubles(P, S, float_rows) * sizeof(double);
+              z.slots * fused_slot_doubles(P, S, float_rows, threads) * sizeof(double);
     return z;
 }
 bool float_rows_of(int precision) {
@@ -1698,7 +1729,9 @@ bool float_rows_of(int precision) {
 // persistent CTA with its penalty rows and its checkpoints (rewritten for every chunk, so it
 // stays in L2) and its group and run sums.
 size_t fused_scratch_bytes(const TraceParams& tp, int P, int precision) {
-    return fused_scratch(tp.V, P, tp.S, make_pieces(tp).count, float_rows_of(precision)).bytes;
+    return fused_scratch(tp.V, P, tp.S, make_pieces(tp).count, float_rows_of(precision),
+                         fused_threads(tp))
+        .bytes;
 }
 
 // The largest over every plan of `tuples` tuples (a piece is whole tuples), every precision and
@@ -1708,13 +1741,54 @@ size_t fused_scratch_bound(int runs, int p_max, int S, int tuples) {
     for (int columns = 1; columns <= fused_np(p_max) / 8; ++columns) {
         const int P = columns * 8 - 1 < p_max ? columns * 8 - 1 : p_max;
         for (int pieces = 1; pieces <= tuples && pieces <= kMaxPieces; ++pieces)
-            for (const bool float_rows : {false, true}) {
-                const size_t b = fused_scratch(runs, P, S, pieces, float_rows).bytes;
-                most = b > most ? b : most;
-            }
+            for (const bool float_rows : {false, true})
+                for (const int threads : {kFusedThreads, kFusedThreadsSmall}) {
+                    if (threads == kFusedThreadsSmall && pieces * 2 * threads > kSmallPlanRays)
+                        continue;  // no such plan
+                    const size_t b =
+                        fused_scratch(runs, P, S, pieces, float_rows, threads).bytes;
+                    most = b > most ? b : most;
+                }
     }
     return most;
 }
+
+namespace {
+using FusedKernel = void (*)(FusedArgs);
+
+template <class N, int kT>
+FusedKernel fused_kernel_of(int feat) {
+    switch (feat) {
+    case 0: return adjoint_gram_kernel<N, 0, kT>;
+    case 1: return adjoint_gram_kernel<N, 1, kT>;
+    case 2: return adjoint_gram_kernel<N, 2, kT>;
+    case 3: return adjoint_gram_kernel<N, 3, kT>;
+    case 4: return adjoint_gram_kernel<N, 4, kT>;
+    case 5: return adjoint_gram_kernel<N, 5, kT>;
+    case 6: return adjoint_gram_kernel<N, 6, kT>;
+    case 8: return adjoint_gram_kernel<N, 8, kT>;
+    case 12: return adjoint_gram_kernel<N, 12, kT>;
+    case 18: return adjoint_gram_kernel<N, 18, kT>;
+    default: return adjoint_gram_kernel<N, 7, kT>;
+    }
+}
+
+template <int kT>
+FusedKernel fused_kernel(int precision, int feat) {
+    switch (precision) {
+    case MKB_PRECISION_FP64: return fused_kernel_of<Exact64, kT>(feat);
+    case MKB_PRECISION_MIXED: return fused_kernel_of<MixedPrecision, kT>(feat);
+    case MKB_PRECISION_FP32_BULK:  // coaxial without plates only
+        switch (feat) {
+        case 4: return adjoint_gram_kernel<BulkPrecision, 4, kT>;
+        case 8: return adjoint_gram_kernel<BulkPrecision, 8, kT>;
+        case 12: return adjoint_gram_kernel<BulkPrecision, 12, kT>;
+        default: return adjoint_gram_kernel<BulkPrecision, 0, kT>;
+        }
+    default: return fused_kernel_of<double, kT>(feat);
+    }
+}
+}  // namespace
 
 int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double* records,
                         double* gram, void* scratch, size_t scratch_bytes, int precision,
@@ -1730,7 +1804,8 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
     const bool float_rows = float_rows_of(precision);
     FusedArgs fa;
     fa.pc = make_pieces(tp);
-    const FusedScratch z = fused_scratch(tp.V, p_max, tp.S, fa.pc.count, float_rows);
+    const int threads = fused_threads(tp);
+    const FusedScratch z = fused_scratch(tp.V, p_max, tp.S, fa.pc.count, float_rows, threads);
     if (scratch == nullptr || scratch_bytes < z.bytes) {
         set_error("fused adjoint: scratch of %zu bytes needed", z.bytes);
         return MKB_ERR_WORKSPACE;
@@ -1744,13 +1819,14 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
     fa.done = fa.queue + 64;
     fa.partial = reinterpret_cast<double*>(static_cast<char*>(scratch) + z.counters);
     fa.scratch = reinterpret_cast<double*>(static_cast<char*>(scratch) + z.counters + z.partial);
-    fa.slot_doubles = fused_slot_doubles(p_max, tp.S, float_rows);
+    fa.slot_doubles = fused_slot_doubles(p_max, tp.S, float_rows, threads);
     fa.run_mask = run_mask;
     fa.order = order;
     fa.vt = rv.table;
     fa.p_max = p_max;
     fa.gram_stride = static_cast<int64_t>(p_max + 1) * (p_max + 1);
-    const size_t smem = fused_adjoint_smem(tp, p_max, float_rows ? sizeof(float) : sizeof(double));
+    const size_t smem = fused_adjoint_smem(tp, p_max, float_rows ? sizeof(float) : sizeof(double),
+                                           threads);
     if (precision == MKB_PRECISION_FP32_BULK && (tp.non_coaxial || tp.G > 0)) {
         set_error("fused adjoint: FP32_BULK is built for coaxial batches without ghost plates");
         return MKB_ERR_UNSUPPORTED;
@@ -1773,40 +1849,9 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
         const int floor_min = rv.table != nullptr ? rv.min_floor : vp.sweep_floor;
         if (floor_min >= plate_max) feat = 18;
     }
-    using Fn = void (*)(FusedArgs);
-    auto pick = [&](auto tag) -> Fn {
-        using N = typename decltype(tag)::type;
-        switch (feat) {
-        case 0: return adjoint_gram_kernel<N, 0>;
-        case 1: return adjoint_gram_kernel<N, 1>;
-        case 2: return adjoint_gram_kernel<N, 2>;
-        case 3: return adjoint_gram_kernel<N, 3>;
-        case 4: return adjoint_gram_kernel<N, 4>;
-        case 5: return adjoint_gram_kernel<N, 5>;
-        case 6: return adjoint_gram_kernel<N, 6>;
-        case 8: return adjoint_gram_kernel<N, 8>;
-        case 12: return adjoint_gram_kernel<N, 12>;
-        default: return adjoint_gram_kernel<N, 7>;
-        }
-    };
-    // FP32_BULK: coaxial without plates only (features 0, 4, 8, 12)
-    auto pick_bulk = [&]() -> Fn {
-        switch (feat) {
-        case 4: return adjoint_gram_kernel<BulkPrecision, 4>;
-        case 8: return adjoint_gram_kernel<BulkPrecision, 8>;
-        case 12: return adjoint_gram_kernel<BulkPrecision, 12>;
-        default: return adjoint_gram_kernel<BulkPrecision, 0>;
-        }
-    };
-    const Fn kernel = feat == 18 ? (precision == MKB_PRECISION_MIXED
-                                          ? adjoint_gram_kernel<MixedPrecision, 18>
-                                      : precision == MKB_PRECISION_FP64
-                                          ? adjoint_gram_kernel<Exact64, 18>
-                                          : adjoint_gram_kernel<double, 18>)
-                      : precision == MKB_PRECISION_FP64    ? pick(TypeTag<Exact64>{})
-                      : precision == MKB_PRECISION_MIXED ? pick(TypeTag<MixedPrecision>{})
-                      : precision == MKB_PRECISION_FP32_BULK ? pick_bulk()
-                                                         : pick(TypeTag<double>{});
+    const FusedKernel kernel = threads == kFusedThreads
+                                   ? fused_kernel<kFusedThreads>(precision, feat)
+                                   : fused_kernel<kFusedThreadsSmall>(precision, feat);
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            static_cast<int>(smem));
     if (err != cudaSuccess) return cuda_status(err, "fused adjoint: shared memory attribute");
@@ -1814,7 +1859,7 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
     err = cudaGetDevice(&device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (err == cudaSuccess)
-        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kFusedThreads, smem);
+        err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
     if (err != cudaSuccess) return cuda_status(err, "fused adjoint: occupancy");
     if (per_sm < 1) {
         set_error("fused adjoint: %zu bytes of shared memory do not fit an SM", smem);
@@ -1827,7 +1872,7 @@ int launch_adjoint_gram(const TraceParams& tp, const VarParams& vp, const double
     if (grid > static_cast<int64_t>(tp.V) * fa.items) grid = tp.V * fa.items;
     err = cudaMemsetAsync(fa.queue, 0, (static_cast<size_t>(tp.V) + 64) * sizeof(int), stream);
     if (err != cudaSuccess) return cuda_status(err, "fused adjoint: clear queue");
-    kernel<<<grid, kFusedThreads, smem, stream>>>(fa);
+    kernel<<<grid, threads, smem, stream>>>(fa);
     count_launch();
     return cuda_status(cudaGetLastError(), "fused adjoint launch");
 }

@@ -2,6 +2,8 @@
 of pieces): one item per run, per group and per piece give every run the same bits, equal to the
 run alone, and [J r]^T [J r] of the materialised Jacobian to the rounding of the sums."""
 
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -61,3 +63,53 @@ def test_the_last_column_tile(surfaces, P):
         d = np.sqrt(np.maximum(np.diagonal(want), 1e-300))
         err = np.abs(gram[v] - want) / (d[:, None] * d[None, :])  # bounds as above
         assert err[:-1, :-1].max() <= 1e-12 and err.max() <= 1e-9
+
+
+# 4,480 rays are 9 pieces on blocks of 256 rays, 2,240 are 8 on blocks of 128. One item per run from
+# eight runs per block of the GPU on, one per group from two: 148 (FP64) and 296 (MIXED) blocks of
+# 256, 444 and 592 of 128, so 1,000 and 1,500 runs are cut into groups in every precision.
+@pytest.mark.parametrize("precision", [PRECISION_FP64, PRECISION_FP64_FMA, PRECISION_MIXED])
+@pytest.mark.parametrize("variants,rings,spokes,items", [
+    (2, 8, 16, 9), (1000, 8, 16, 4), (4200, 8, 16, 1),
+    (3, 4, 16, 8), (1500, 4, 16, 4), (5000, 4, 16, 1),
+    (3, 5, 11, 4),   # 55 rays per tuple: pieces of 495, the last of 440
+    (5, 1, 8, 1),    # 280 rays, one piece
+    (2, 1, 4, 1),    # 140 rays, a chunk and a part
+])
+def test_items_per_run_and_their_sums(monkeypatch, variants, rings, spokes, items, precision):
+    """The split that the batch size asks for is the one taken (the runs' item counters, after the
+    records and the queue counter in the workspace), and its sums are the run's alone."""
+    b, st, vs, x0 = workloads.sweep(variants, surfaces=6, wavelengths=7, rings=rings,
+                                    spokes=spokes, precision=precision)
+    lay = ResidualLayout(b.topology, st)
+    db = engine.DeviceSystemBatch(b)
+    made, empty = [], torch.empty
+
+    def keep(*args, **kwargs):
+        made.append(empty(*args, **kwargs))
+        return made[-1]
+    monkeypatch.setattr(torch, "empty", keep)
+    gram = engine.adjoint_normal_equations_device(db, lay, b, vs, x0)
+    monkeypatch.undo()
+    torch.cuda.synchronize()
+    ws = next(t for t in made if t.dtype == torch.uint8)
+    at = -(-8 * variants * db.stride // 256) * 256 + 256
+    done = ws[at:at + 4 * variants].view(torch.int32)
+    assert (done == (items if items > 1 else 0)).all()
+    for v in sorted({0, variants // 2, variants - 1}):
+        one = b.take([v])
+        alone = engine.adjoint_normal_equations_device(engine.DeviceSystemBatch(one), lay, one, vs,
+                                                       x0[v:v + 1])
+        assert torch.equal(gram[v], alone[0]), v
+        J, r, _ = engine.adjoint_jacobian_device(
+            engine.DeviceSystemBatch(one),
+            ResidualLayout(b.topology, dataclasses.replace(st, precision=PRECISION_FP64)), one, vs,
+            x0[v:v + 1])
+        X = np.concatenate([J[0].cpu().numpy(), r[0].cpu().numpy()[None]])
+        want = X @ X.T
+        d = np.sqrt(np.maximum(np.diagonal(want), 1e-300))
+        err = np.abs(gram[v].cpu().numpy() - want) / (d[:, None] * d[None, :])
+        if precision == PRECISION_MIXED:  # FP32 rows: every entry within 2e-3
+            assert err.max() <= 2e-3
+        else:  # bounds as above
+            assert err[:-1, :-1].max() <= 1e-12 and err.max() <= 1e-9

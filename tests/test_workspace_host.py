@@ -1,7 +1,7 @@
 """Sizes of the adjoint workspaces (host functions, no GPU): a call asks for what its plan and
-variables can use -- a block of 256 rays in the fused adjoint keeps (columns + 10 S) values per ray
-and two sums of its tile pairs, a block of 128 rays of the Jacobian 10 S + 1 -- and the sizes that
-are asked for without a plan suit every plan."""
+variables can use -- a block of 256 rays in the fused adjoint (128 in plans of at most 3,072 rays)
+keeps (columns + 10 S) values per ray and two sums of its tile pairs, a block of 128 rays of the
+Jacobian 10 S + 1 -- and the sizes that are asked for without a plan suit every plan."""
 
 import ctypes as C
 import dataclasses
@@ -24,17 +24,19 @@ def _case(make, precision, **kw):
     return b, lay.plan(b), shape, vs
 
 
-def _pieces(b, rays_per_tuple):
-    """Whole tuples of at least 512 rays (every field of these cases has the same pupil)."""
-    tuples = b.fields * b.wavelengths
-    target = max(512, -(-tuples * rays_per_tuple // 64))
-    per = -(-target // rays_per_tuple)
-    return -(-tuples // per)
+def _fused(b, plan, precision):
+    """Threads of a block, blocks at most, and the most pieces of a run: whole tuples, two blocks of
+    rays or more (but for a last piece in plans of many rays)."""
+    rays = int(_capi.lib().mkb_rays_per_variant(C.byref(plan)))
+    threads = 128 if rays <= 3072 else 256
+    mixed = precision == PRECISION_MIXED
+    blocks = SMS * ((4 if mixed else 3) if threads == 128 else (2 if mixed else 1))
+    return threads, blocks, min(b.fields * b.wavelengths, -(-rays // (2 * threads)))
 
 
-def _slot(P, S, precision):
+def _slot(P, S, precision, threads):
     cols = (P + 8) // 8
-    values = (8 * cols + 10 * S) * 256 * (4 if precision == PRECISION_MIXED else 8)
+    values = (8 * cols + 10 * S) * threads * (4 if precision == PRECISION_MIXED else 8)
     return values, cols * (cols + 1) // 2 * 512
 
 
@@ -42,6 +44,7 @@ CASES = [
     (workloads.singlet, {}),
     (workloads.sweep, dict(surfaces=30, wavelengths=7, rings=16, spokes=32)),
     (workloads.sweep, dict(surfaces=43, wavelengths=2, rings=3, spokes=5)),
+    (workloads.sweep, dict(surfaces=10, wavelengths=7, rings=6, spokes=12)),
 ]
 
 
@@ -51,13 +54,11 @@ CASES = [
 def test_fused_workspace_holds_what_the_items_use(make, kw, precision, runs):
     lib = _capi.lib()
     b, plan, shape, vs = _case(make, precision, **kw)
-    rays = int(lib.mkb_rays_per_variant(C.byref(plan))) // (b.fields * b.wavelengths)
-    pieces = _pieces(b, rays)
+    threads, ctas, pieces = _fused(b, plan, precision)
     v = vs.c_struct()
     need = int(lib.mkb_adjoint_normal_equations_workspace_bytes(C.byref(shape), C.byref(plan),
                                                                 C.byref(v), 0, runs))
-    values, sums = _slot(vs.size, b.surfaces, precision)
-    ctas = SMS * (2 if precision == PRECISION_MIXED else 1)
+    values, sums = _slot(vs.size, b.surfaces, precision, threads)
     assert need >= 8 * runs * shape.record_stride + (values + 2 * sums)  # a block at least
     # records, counters, the items' sums, the blocks' states; three parts are rounded up to 256
     assert need <= (8 * runs * shape.record_stride + 4 * (runs + 64) + 3 * 256 +
