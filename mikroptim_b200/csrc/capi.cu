@@ -131,8 +131,8 @@ int residual_scales(const mkb_residual_plan* plan, double* scale) {
     return MKB_OK;
 }
 
-int make_trace_params(const mkb_device_batch* batch, const mkb_residual_plan* plan,
-                      int pack_rays, TraceParams* out) {
+int make_trace_shape(const mkb_device_batch* batch, const mkb_residual_plan* plan,
+                     TraceParams* out) {
     if (batch == nullptr) {
         set_error("batch is null");
         return MKB_ERR_ARGUMENT;
@@ -258,6 +258,17 @@ int make_trace_params(const mkb_device_batch* batch, const mkb_residual_plan* pl
         offset += L * p.sample_count[f];
     }
     p.rays = offset;
+    p.n_tuples = F * L;
+    p.transverse = plan->transverse_weight > 0.0 ? 1 : 0;
+    return MKB_OK;
+}
+
+int make_trace_params(const mkb_device_batch* batch, const mkb_residual_plan* plan,
+                      int pack_rays, TraceParams* out) {
+    const int rc = make_trace_shape(batch, plan, out);
+    if (rc != MKB_OK) return rc;
+    TraceParams& p = *out;
+    const int L = p.L, F = p.F;
     // pupil tables (pupil/quadrature.hpp:71): rho = sqrt(u), weight = W / M, phi per mode
     const double pi = 3.14159265358979323846264338327950288;
     for (int i = 0; i < plan->rings; ++i) {
@@ -275,7 +286,6 @@ int make_trace_params(const mkb_device_batch* batch, const mkb_residual_plan* pl
         p.sin_full[j] = std::sin(full);
         p.cos_full[j] = std::cos(full);
     }
-    p.n_tuples = F * L;
     const double lambda_ref_mm = plan->reference_wavelength_nm * 1e-6;
     for (int f = 0; f < F; ++f)
         for (int l = 0; l < L; ++l) {
@@ -284,7 +294,6 @@ int make_trace_params(const mkb_device_batch* batch, const mkb_residual_plan* pl
             p.pscale[f * L + l] = w > 0.0 ? std::sqrt(plan->fail_weight * w) : 0.0;
             p.tscale[f * L + l] = w > 0.0 ? std::sqrt(plan->transverse_weight * w) : 0.0;
         }
-    p.transverse = plan->transverse_weight > 0.0 ? 1 : 0;
     // pack plan: consecutive tuples until pack_rays rays or kMaxPackTuples tuples; a tuple
     // with more rays than pack_rays (fine pupils) gets a pack of its own
     for (int t = 0; t < p.n_tuples; ++t)

@@ -1007,6 +1007,10 @@ int residual_scales(const mkb_residual_plan* plan, double* scale);
 
 // Builds the parameter block from the batch and plan; returns MKB_OK or MKB_ERR_ARGUMENT.
 // `pack_rays` = rays one CTA traces (tuples are packed until this many rays).
+// make_trace_shape: the checks, and of *out the shape alone (what sizes depend on), without the
+// pupil tables, the scales and the packs
+int make_trace_shape(const mkb_device_batch* batch, const mkb_residual_plan* plan,
+                     TraceParams* out);
 int make_trace_params(const mkb_device_batch* batch, const mkb_residual_plan* plan,
                       int pack_rays, TraceParams* out);
 

@@ -445,7 +445,7 @@ size_t mkb_adjoint_jacobian_plan_workspace_bytes(const mkb_device_batch* templat
     TraceParams tp;
     mkb_device_batch b = *templates;
     b.variants = runs;
-    if (make_trace_params(&b, plan, pack_rays_default(), &tp) != MKB_OK) return 0;
+    if (make_trace_shape(&b, plan, &tp) != MKB_OK) return 0;
     return jacobian_bytes(tp);
 }
 
@@ -538,7 +538,7 @@ size_t mkb_adjoint_normal_equations_workspace_bytes(const mkb_device_batch* temp
     TraceParams tp;
     mkb_device_batch b = *templates;
     b.variants = runs;
-    if (make_trace_params(&b, plan, pack_rays_default(), &tp) != MKB_OK) return 0;
+    if (make_trace_shape(&b, plan, &tp) != MKB_OK) return 0;
     return normal_equations_bytes(tp, pmax, plan->precision, per_run_variables != 0);
 }
 
