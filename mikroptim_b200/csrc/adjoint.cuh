@@ -74,7 +74,7 @@ __device__ __forceinline__ void adjoint_from_surface(const Transform<A>& t, RayA
 // A divisor of the adjoint arithmetic. FP32 (the mixed sweep): the SFU reciprocal, taken once
 // per step and shared by the K seeds, and a multiply -- a few ulp of single precision, inside
 // that sweep's rounding budget. FP64: the rounded division in the reference's order, so the
-// FP64 sweeps stay bit-identical.
+// materialised rows stay bit-identical (the fused sweeps take ReciprocalDivisor).
 __device__ __forceinline__ float sfu_reciprocal(float x) { return __fdividef(1.0f, x); }
 
 template <class A>
@@ -94,13 +94,15 @@ struct Divisor<float> {
 // alone, is divided ahead of the adjoints' dependent chain, and a quotient on that chain is a
 // multiply and one correction by its exact remainder. With a correctly rounded reciprocal the
 // corrected quotient is the rounded one (P. Markstein, IBM J. Res. Dev. 34, 1990) except where
-// the remainder underflows, for a reciprocal of infinity (the uncorrected quotient is returned)
-// and for the sign of a zero.
+// the remainder underflows (a dividend below 2^-914, a subnormal quotient: within one unit of the
+// last place), for the sign of a zero, and for subnormal divisors, whose reciprocal overflows: the
+// sweeps divide by refractive indices, direction cosines and roots of the refraction, which are
+// not. (Host code too: a test compares it with the division.)
 template <class A>
 struct ReciprocalDivisor {
     A d, r;
-    __device__ __forceinline__ explicit ReciprocalDivisor(A x) : d(x), r(A(1.0) / x) {}
-    __device__ __forceinline__ A div(A a) const {
+    __host__ __device__ __forceinline__ explicit ReciprocalDivisor(A x) : d(x), r(A(1.0) / x) {}
+    __host__ __device__ __forceinline__ A div(A a) const {
         const double x = value_of(d), y = value_of(r), q = value_of(a) * y;
         const double c = fma(fma(-x, q, value_of(a)), y, q);
         return A(c == c ? c : q);

@@ -405,7 +405,7 @@ __device__ __forceinline__ Exact32 nsqrt(Exact32 a) { return __fsqrt_rn(a.v); }
 __device__ __forceinline__ float value_of(Exact32 a) { return a.v; }
 __device__ __forceinline__ double nsqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ float nsqrt(float a) { return sqrtf(a); }
-__device__ __forceinline__ double value_of(double a) { return a; }
+__host__ __device__ __forceinline__ double value_of(double a) { return a; }
 __device__ __forceinline__ double value_of(Exact64 a) { return a.v; }
 __device__ __forceinline__ float value_of(float a) { return a; }
 
