@@ -566,7 +566,7 @@ constexpr int kMaxTilePairs = kMaxTileCols * (kMaxTileCols + 1) / 2;            
 // of kept_rows_kernel
 constexpr int kFusedSms = 148;
 constexpr int kMaxRowsSlots = 148 * kRowsMinBlocks;
-// Pieces of a run (make_pieces): two to four blocks of rays each, at most kPieceGroups groups of
+// Pieces of a run (make_pieces): a few blocks of rays each, at most kPieceGroups groups of
 // consecutive pieces. Two blocks of 256 rays are about 0.1 ms of one CTA, against some 2 us to
 // stage a record and store a piece's sum.
 constexpr int kMaxPieces = 64;
@@ -1096,14 +1096,16 @@ int fused_threads(const TraceParams& p) {
 
 // Pieces of whole tuples and of at least two blocks of rays, more when a run would otherwise have
 // more than kMaxPieces. In plans of few rays a block left mostly idle is a large part of the run:
-// there no piece is shorter, and of the ends up to four blocks the first is taken that leaves at
-// most 1/16 of its blocks' threads idle, else the one that leaves the fewest (4,096 systems of
-// 15 tuples of 48 rays, FP64: 2,230 us with the first end, 2,010 us so).
+// pieces are one and a half to four blocks there, none is shorter, and of the ends in that range the
+// first is taken that leaves at most 1/16 of its blocks' threads idle, else the one that leaves the
+// fewest (4,096 systems of 15 tuples of 48 rays, FP64: 2,230 us with the first end of two blocks,
+// 2,010 us so).
 FusedPieces make_pieces(const TraceParams& p) {
     FusedPieces c{};
     const int block = fused_threads(p), least = (p.rays + kMaxPieces - 1) / kMaxPieces;
-    const int low = 2 * block > least ? 2 * block : least;
     const bool first = block == kFusedThreads;
+    const int blocks2 = first ? 4 : 3;  // half blocks of the smallest piece
+    const int low = blocks2 * block / 2 > least ? blocks2 * block / 2 : least;
     int t = 0, ray = 0;
     while (t < p.n_tuples) {
         c.ray[c.count++] = ray;
@@ -1112,9 +1114,9 @@ FusedPieces make_pieces(const TraceParams& p) {
         for (int e = t; e < p.n_tuples && idle > 1.0 / 16.0; ++e) {
             have += p.sample_count[e / p.L];
             if (have < low) continue;
-            if (!first &&
-                (p.rays - ray - have < low || (have >= 2 * low && idle < 1.0)))
-                break;
+            const int rest = p.rays - ray - have;
+            if (!first && rest != 0 && rest < low) continue;
+            if (have > 4 * block && idle < 1.0) break;
             const int blocks = (have + block - 1) / block;
             const double share = 1.0 - static_cast<double>(have) / (blocks * block);
             if (share < idle) {
@@ -1743,7 +1745,7 @@ size_t fused_scratch_bound(int runs, int p_max, int S, int tuples) {
         for (int pieces = 1; pieces <= tuples && pieces <= kMaxPieces; ++pieces)
             for (const bool float_rows : {false, true})
                 for (const int threads : {kFusedThreads, kFusedThreadsSmall}) {
-                    if (threads == kFusedThreadsSmall && pieces * 2 * threads > kSmallPlanRays)
+                    if (threads == kFusedThreadsSmall && pieces * 3 * threads / 2 > kSmallPlanRays)
                         continue;  // no such plan
                     const size_t b =
                         fused_scratch(runs, P, S, pieces, float_rows, threads).bytes;

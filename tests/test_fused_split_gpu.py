@@ -65,14 +65,14 @@ def test_the_last_column_tile(surfaces, P):
         assert err[:-1, :-1].max() <= 1e-12 and err.max() <= 1e-9
 
 
-# 4,480 rays are 9 pieces on blocks of 256 rays, 2,240 are 8 on blocks of 128. One item per run from
+# 4,480 rays are 9 pieces on blocks of 256 rays, 2,240 are 9 on blocks of 128. One item per run from
 # eight runs per block of the GPU on, one per group from two: 148 (FP64) and 296 (MIXED) blocks of
 # 256, 444 and 592 of 128, so 1,000 and 1,500 runs are cut into groups in every precision.
 @pytest.mark.parametrize("precision", [PRECISION_FP64, PRECISION_FP64_FMA, PRECISION_MIXED])
 @pytest.mark.parametrize("variants,rings,spokes,items", [
     (2, 8, 16, 9), (1000, 8, 16, 4), (4200, 8, 16, 1),
-    (3, 4, 16, 8), (1500, 4, 16, 4), (5000, 4, 16, 1),
-    (3, 5, 11, 4),   # 55 rays per tuple: pieces of 495, the last of 440
+    (3, 4, 16, 9), (1500, 4, 16, 4), (5000, 4, 16, 1),
+    (3, 5, 11, 5),   # 55 rays per tuple: pieces of 495, the last two of 220
     (5, 1, 8, 1),    # 280 rays, one piece
     (2, 1, 4, 1),    # 140 rays, a chunk and a part
 ])

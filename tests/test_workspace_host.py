@@ -25,13 +25,13 @@ def _case(make, precision, **kw):
 
 
 def _fused(b, plan, precision):
-    """Threads of a block, blocks at most, and the most pieces of a run: whole tuples, two blocks of
-    rays or more (but for a last piece in plans of many rays)."""
+    """Threads of a block, blocks at most, and the most pieces of a run: whole tuples of at least 192
+    rays (plans of few rays) or 512 (but for the last piece)."""
     rays = int(_capi.lib().mkb_rays_per_variant(C.byref(plan)))
     threads = 128 if rays <= 3072 else 256
     mixed = precision == PRECISION_MIXED
     blocks = SMS * ((4 if mixed else 3) if threads == 128 else (2 if mixed else 1))
-    return threads, blocks, min(b.fields * b.wavelengths, -(-rays // (2 * threads)))
+    return threads, blocks, min(b.fields * b.wavelengths, -(-rays // (192 if threads == 128 else 512)))
 
 
 def _slot(P, S, precision, threads):
