@@ -6,7 +6,7 @@
 //     order, acc = fma(u_r, v_r, acc) from acc = 0: bit-identical to the reference's
 //     normal_equations_host / gram_dot (include/mikroptim/optim/normal_equations.hpp:19,33).
 //     One CTA per run and pair of column tiles streams row tiles through shared memory; each
-//     thread advances four chains.
+//     thread advances four chains (one in batches of at most eight columns).
 //   gram_dmma_kernel -- FP64 tensor cores: mma.sync.m8n8k4 (f64) on 8 x 8 output tiles of the
 //     upper triangle, row tiles of J staged in shared memory; fixed k order (deterministic, not
 //     bit-identical to the chain). gram_one_tile_kernel: at most eight columns, no staging.
@@ -18,11 +18,9 @@ namespace {
 
 constexpr int kGramThreads = 256;
 constexpr int kMaxCols = MKB_MAX_VARIABLES + 1;
-// exact kernel: threads, columns of a tile, rows of a staged tile, stages, column stride
+// exact kernel: threads, rows of a staged tile, column stride
 constexpr int kExactThreads = 64;
-constexpr int kExactCols = 16;
 constexpr int kExactRows = 32;
-constexpr int kExactStages = 4;
 constexpr int kExactLd = kExactRows + 2;
 
 // Column c of run `run`: J columns are strided by `stride` per run (the largest P of an uneven
@@ -46,20 +44,31 @@ __device__ __forceinline__ void copy_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
 }
 
-// One CTA per run and pair of 16-column tiles (ta <= tb); thread (ti, tj) advances the four
-// chains of columns {ti, ti + 8} x {tj, tj + 8}, so a row costs it four shared loads for four
+// One CTA per run and pair of 8 kSub-column tiles (ta <= tb); thread (ti, tj) advances the kSub^2
+// chains of columns {ti, ti + 8} x {tj, tj + 8}, so a row costs it 2 kSub shared loads for kSub^2
 // multiply-adds, eight rows' loads ahead of their use. Row tiles come in by 8-byte cp.async (a
-// column starts at any multiple of R), kExactStages deep. What bounds it is the chain itself, R
+// column starts at any multiple of R), kStages deep. What bounds it is the chain itself, R
 // dependent multiply-adds, and the shared loads beside it. The column stride of 17 16-byte units
 // keeps the two-row loads of eight neighbouring columns on different banks. 48 runs of P = 29 and
 // 28,896 rows: one CTA per run with one chain per pair and synchronous tiles took 2,975 us, four
 // chains a thread loaded as they go 1,445 us, 128 threads of two chains with loads ahead 525 us,
 // this 455 us.
+// kSub = 1 for batches of at most eight columns, where three of four chains would be no one's.
+// kPacked: for more CTAs than fit the GPU at once. Three stages instead of four (which hide the
+// loads better) let seven CTAs of kSub = 2 reside on an SM instead of six. And a last tile of at
+// most kTail columns, which leaves half the threads of its pairs idle, has its own chains done by
+// them in pair (0, tb), so that pair (tb, tb) does nothing. One CTA per run / kSub = 2 and nothing
+// packed / now (us): 512 runs of 900 rows, P = 6 24.7 / 28.7 / 17.2, P = 16 56.9 / 70.0 / 55.4;
+// 16,384 runs of 35 rows, P = 16 137 / 157 / 114, P = 64 866 / 901 / 748.
+constexpr int kTail = 4;
+constexpr int kFewExactCtas = 148 * 6;  // that fit at once with four stages
+template <int kSub, bool kPacked>
 __global__ void __launch_bounds__(kExactThreads)
 gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, int P_all,
                   int64_t R, double* __restrict__ gram, const int* __restrict__ run_mask,
                   const VarParams* __restrict__ vt, int stride, int tile_pairs) {
-    __shared__ __align__(16) double tile[kExactStages][2 * kExactCols * kExactLd];
+    constexpr int kCols = 8 * kSub, kStages = kPacked ? 3 : 4;
+    __shared__ __align__(16) double tile[kStages][2 * kCols * kExactLd];
     // grid (runs, tile pairs), walked so that the pairs of a run are neighbours (their columns
     // are in L2 once)
     const int64_t block = static_cast<int64_t>(blockIdx.y) * gridDim.x + blockIdx.x;
@@ -69,12 +78,14 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
     while (ta > tb) ta -= ++tb;  // pair index -> (ta, tb), column by column of the triangle
     const int P = vt != nullptr ? vt[run].P : P_all;
     const int n = P + 1;
-    if (tb * kExactCols >= n) return;
+    if (tb * kCols >= n) return;
     const bool diagonal = ta == tb;
+    const bool tail = kPacked && tb > 0 && n - tb * kCols <= kTail;
+    if (diagonal && tail) return;
     const int tid = threadIdx.x, ti = tid >> 3, tj = tid & 7;
     // this thread's row of every staged tile and the columns it copies; columns past n and rows
     // past R are filled with zeros
-    constexpr int kCopies = 2 * kExactCols * kExactRows / kExactThreads;
+    constexpr int kCopies = 2 * kCols * kExactRows / kExactThreads;
     constexpr int kCopyStep = kExactThreads / kExactRows;
     const int copies = diagonal ? kCopies / 2 : kCopies;
     const int k_in = tid & (kExactRows - 1), c_in = tid / kExactRows;
@@ -83,13 +94,13 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
 #pragma unroll
     for (int i = 0; i < kCopies; ++i) {
         const int c = c_in + i * kCopyStep;
-        const int col = c < kExactCols ? ta * kExactCols + c : tb * kExactCols + c - kExactCols;
+        const int col = c < kCols ? ta * kCols + c : tb * kCols + c - kCols;
         in[i] = col < n && i < copies;
         src[i] = in[i] ? column(J, r, run, col, P, stride, R) + k_in : r;
     }
     auto load = [&](int64_t step) {
         const int64_t r0 = step * kExactRows;
-        double* dst = tile[step % kExactStages] + c_in * kExactLd + k_in;
+        double* dst = tile[step % kStages] + c_in * kExactLd + k_in;
         const bool row = r0 + k_in < R;
 #pragma unroll
         for (int i = 0; i < kCopies; ++i)
@@ -98,35 +109,41 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
                             in[i] && row);
     };
     const int64_t steps = (R + kExactRows - 1) / kExactRows;
-    for (int s = 0; s < kExactStages - 1; ++s) {
+    for (int s = 0; s < kStages - 1; ++s) {
         if (s < steps) load(s);
         copy_async_commit();
     }
     // chains {p, p + 8} x {q, q + 8}; on the diagonal (p + 8, q) is the transposed pair's
-    const int p = ta * kExactCols + ti, q = tb * kExactCols + tj;
-    const bool mine = p < n && q < n && (!diagonal || ti <= tj);
-    const int u_at = ti * kExactLd, v_at = (diagonal ? tj : kExactCols + tj) * kExactLd;
+    const bool own = tail && ta == 0 && tj >= kTail;  // one of the tail's own chains
+    const int p = (own ? tb : ta) * kCols + ti, q = tb * kCols + tj - (own ? kTail : 0);
+    const bool mine = p < n && q < n && (!(diagonal || own) || p <= q);
+    const int u_at = (own ? kCols + ti : ti) * kExactLd;
+    const int v_at = (diagonal ? tj : kCols + tj - (own ? kTail : 0)) * kExactLd;
     constexpr int kNext = 8 * kExactLd;
-    double a00 = 0.0, a01 = 0.0, a10 = 0.0, a11 = 0.0;
+    double acc[kSub][kSub] = {};
     for (int64_t step = 0; step < steps; ++step) {
-        copy_async_wait<kExactStages - 2>();
+        copy_async_wait<kStages - 2>();
         __syncthreads();  // this step's rows are here; the slot of the last one is free
-        if (step + kExactStages - 1 < steps) load(step + kExactStages - 1);
+        if (step + kStages - 1 < steps) load(step + kStages - 1);
         copy_async_commit();
         if (!mine) continue;
-        const double* u = tile[step % kExactStages] + u_at;
-        const double* v = tile[step % kExactStages] + v_at;
+        const double* u = tile[step % kStages] + u_at;
+        const double* v = tile[step % kStages] + v_at;
         const int64_t left = R - step * kExactRows;
         if (left >= kExactRows) {
             // eight rows' loads ahead of their chains
-            double2 u0[2][4], u1[2][4], v0[2][4], v1[2][4];
+            double2 x[2][kSub][4], y[2][kSub][4];
             auto fetch = [&](int k, int h) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    u0[h][i] = *reinterpret_cast<const double2*>(u + k + 2 * i);
-                    u1[h][i] = *reinterpret_cast<const double2*>(u + kNext + k + 2 * i);
-                    v0[h][i] = *reinterpret_cast<const double2*>(v + k + 2 * i);
-                    v1[h][i] = *reinterpret_cast<const double2*>(v + kNext + k + 2 * i);
+#pragma unroll
+                    for (int c = 0; c < kSub; ++c)
+                        x[h][c][i] =
+                            *reinterpret_cast<const double2*>(u + c * kNext + k + 2 * i);
+#pragma unroll
+                    for (int c = 0; c < kSub; ++c)
+                        y[h][c][i] =
+                            *reinterpret_cast<const double2*>(v + c * kNext + k + 2 * i);
                 }
             };
             fetch(0, 0);
@@ -136,32 +153,31 @@ gram_exact_kernel(const double* __restrict__ J, const double* __restrict__ r, in
                 if (k + 8 < kExactRows) fetch(k + 8, h ^ 1);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    a00 = fma(u0[h][i].x, v0[h][i].x, a00);
-                    a01 = fma(u0[h][i].x, v1[h][i].x, a01);
-                    a10 = fma(u1[h][i].x, v0[h][i].x, a10);
-                    a11 = fma(u1[h][i].x, v1[h][i].x, a11);
-                    a00 = fma(u0[h][i].y, v0[h][i].y, a00);
-                    a01 = fma(u0[h][i].y, v1[h][i].y, a01);
-                    a10 = fma(u1[h][i].y, v0[h][i].y, a10);
-                    a11 = fma(u1[h][i].y, v1[h][i].y, a11);
+#pragma unroll
+                    for (int e = 0; e < kSub * kSub; ++e)
+                        acc[e / kSub][e % kSub] = fma(x[h][e / kSub][i].x, y[h][e % kSub][i].x,
+                                                      acc[e / kSub][e % kSub]);
+#pragma unroll
+                    for (int e = 0; e < kSub * kSub; ++e)
+                        acc[e / kSub][e % kSub] = fma(x[h][e / kSub][i].y, y[h][e % kSub][i].y,
+                                                      acc[e / kSub][e % kSub]);
                 }
             }
         } else {
             for (int k = 0; k < left; ++k) {
-                a00 = fma(u[k], v[k], a00);
-                a01 = fma(u[k], v[kNext + k], a01);
-                a10 = fma(u[kNext + k], v[k], a10);
-                a11 = fma(u[kNext + k], v[kNext + k], a11);
+#pragma unroll
+                for (int e = 0; e < kSub * kSub; ++e)
+                    acc[e / kSub][e % kSub] = fma(u[e / kSub * kNext + k], v[e % kSub * kNext + k],
+                                                  acc[e / kSub][e % kSub]);
             }
         }
     }
     if (!mine) return;
     double* g = gram + run * (stride + 1) * (stride + 1);
-    const double acc[2][2] = {{a00, a01}, {a10, a11}};
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kSub; ++i) {
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < kSub; ++j) {
             const int c = p + 8 * i, d = q + 8 * j;
             if (c >= n || d >= n) continue;
             g[static_cast<int64_t>(d) * n + c] = acc[i][j];
@@ -189,7 +205,7 @@ __device__ inline void dmma_8x8x4(double& d0, double& d1, double a, double b) {
 // same entries (lane l: column l / 4, row l % 4), so every warp streams its own rows straight from
 // memory, 32 bytes of each column at a time, and the eight warps' sums are added in order. The
 // tiles below leave seven warps idle here and wait for a tile at a time; 1,024 runs of P = 4 and
-// 900 rows: 45.8 us there, 10.2 us here. Which way a run goes is decided by its own P alone, so
+// 900 rows, in L2: 32.5 us there, 6.7 us here. Which way a run goes is decided by its own P alone, so
 // that its bits are the same in every batch. part: [kDmmaWarps * 64] in shared memory.
 __device__ __forceinline__ void one_tile_sums(const double* J, const double* r, int64_t run, int P,
                                               int stride, int64_t R, double* part, double* gram) {
@@ -318,11 +334,15 @@ int launch_gram(const double* J, const double* r, int runs, int P, int64_t R, do
     if (runs <= 0) return MKB_OK;
     const int stride = rv.table != nullptr ? rv.stride : P;
     if (exact) {
-        const int tiles = (stride + 1 + kExactCols - 1) / kExactCols;
+        const int tiles = stride + 1 <= 8 ? 1 : (stride + 1 + 15) / 16;
         const int tile_pairs = tiles * (tiles + 1) / 2;
         const dim3 grid(static_cast<unsigned>(runs), static_cast<unsigned>(tile_pairs));
-        gram_exact_kernel<<<grid, kExactThreads, 0, stream>>>(J, r, P, R, gram, run_mask, rv.table,
-                                                              stride, tile_pairs);
+        const bool few = static_cast<int64_t>(runs) * tile_pairs <= kFewExactCtas;
+        auto kernel = stride + 1 <= 8 ? gram_exact_kernel<1, true>
+                      : few           ? gram_exact_kernel<2, false>
+                                      : gram_exact_kernel<2, true>;
+        kernel<<<grid, kExactThreads, 0, stream>>>(J, r, P, R, gram, run_mask, rv.table, stride,
+                                                   tile_pairs);
     } else if (stride + 1 <= 8)
         gram_one_tile_kernel<<<runs, kGramThreads, 0, stream>>>(J, r, P, R, gram, run_mask,
                                                                 rv.table, stride);

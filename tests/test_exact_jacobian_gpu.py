@@ -27,6 +27,14 @@ def test_chains_equal_the_oracle(P, rows):
         assert np.array_equal(got[i], got[i].T)
 
 
+@pytest.mark.parametrize("P", [2, 6, 8, 17, 18, 19, 20, 23, 34, 35, 36, 50])
+@pytest.mark.parametrize("rows", [35, 96, 100])
+def test_chains_of_narrow_and_last_tiles_equal_the_oracle(P, rows):
+    """One chain per thread up to eight columns; one to four columns in the last tile of sixteen,
+    whose own chains the pair with the first tile takes, and five."""
+    test_chains_equal_the_oracle(P, rows)
+
+
 @pytest.mark.parametrize("P", [1, 4, 7, 8])
 @pytest.mark.parametrize("rows", [1, 3, 127, 128, 129, 900])
 def test_tensor_core_sums_of_few_columns(P, rows):

@@ -69,7 +69,8 @@ def test_uneven_lm_equals_each_run_alone(method):
     assert np.all(together["merit"] <= together["history"][:, 0])
 
 
-def test_uneven_fd_lm_of_narrow_and_wide_runs_equals_each_run_alone():
+@pytest.mark.parametrize("exact", [False, True])
+def test_uneven_fd_lm_of_narrow_and_wide_runs_equals_each_run_alone(exact):
     """Runs of at most seven variables beside wider ones: their FD normal equations are summed in
     the order they are summed in alone."""
     b, st, vss, x0 = workloads.uneven(8, rings=4, spokes=8, p_min=4, p_max=11,
@@ -77,7 +78,7 @@ def test_uneven_fd_lm_of_narrow_and_wide_runs_equals_each_run_alone():
     P = np.array([v.size for v in vss])
     assert (P <= 7).sum() >= 2 and (P >= 8).sum() >= 2
     lay = ResidualLayout(b.topology, st)
-    opt = engine.LmOptions(max_iterations=12, gram_exact=False, jacobian=engine.JACOBIAN_FD)
+    opt = engine.LmOptions(max_iterations=12, gram_exact=exact, jacobian=engine.JACOBIAN_FD)
     together = engine.optimize_lm_gpu(b, lay, vss, x0, opt)
     for v in range(b.variants):
         one = workloads.unpad(b, v)
