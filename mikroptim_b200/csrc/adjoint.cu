@@ -380,52 +380,52 @@ projection_kernel(const __grid_constant__ AdjointParams ap, const uint8_t* __res
     const TraceParams& p = ap.t;
     const int P = ap.v.P;
     for (int64_t rt = blockIdx.x; rt < total; rt += gridDim.x) {
-    const int64_t run = rt / p.n_tuples;
-    const int tu = static_cast<int>(rt - run * p.n_tuples);
-    const int f = tu / p.L;
-    const int l = tu - f * p.L;
-    const int n = p.sample_count[f];
-    const int64_t row0 = p.field_offset[f] + static_cast<int64_t>(l) * n;
-    const uint8_t* st = status + run * p.rays + row0;
-    double* col0 = J + run * P * ap.rows + row0;
-    const int mode = p.pupil_mode[f];
-    const int M = mode == MKB_PUPIL_AXIS ? 1 : p.spokes;
-    const double* w_tab = mode == MKB_PUPIL_AXIS ? p.w_axis : p.w_spoke;
-    const double* rw_tab = mode == MKB_PUPIL_AXIS ? p.rw_axis : p.rw_spoke;
-    const int tid = threadIdx.x, k_in = tid % kProjRows, c_in = tid / kProjRows;
-    constexpr int kColStep = kProjThreads / kProjRows;
-    N sum(0.0);
-    for (int base = 0; base < n; base += kProjRows) {
-        const int k = base + k_in;
-        const bool in = k < n && in_piston(st[k]);
-        const N w = in ? N(w_tab[k / M]) : N(0.0);
-        for (int c = c_in; c < P; c += kColStep)
-            term[c * kProjLd + k_in] = in ? value_of(w * N(col0[c * ap.rows + k])) : 0.0;
-        if (c_in == 0) term[P * kProjLd + k_in] = value_of(w);
-        __syncthreads();
-        if (tid <= P) {
-            const int rows = n - base < kProjRows ? n - base : kProjRows;
-            const double* t = term + tid * kProjLd;
-            for (int i = 0; i < rows; ++i) sum += N(t[i]);
+        const int64_t run = rt / p.n_tuples;
+        const int tu = static_cast<int>(rt - run * p.n_tuples);
+        const int f = tu / p.L;
+        const int l = tu - f * p.L;
+        const int n = p.sample_count[f];
+        const int64_t row0 = p.field_offset[f] + static_cast<int64_t>(l) * n;
+        const uint8_t* st = status + run * p.rays + row0;
+        double* col0 = J + run * P * ap.rows + row0;
+        const int mode = p.pupil_mode[f];
+        const int M = mode == MKB_PUPIL_AXIS ? 1 : p.spokes;
+        const double* w_tab = mode == MKB_PUPIL_AXIS ? p.w_axis : p.w_spoke;
+        const double* rw_tab = mode == MKB_PUPIL_AXIS ? p.rw_axis : p.rw_spoke;
+        const int tid = threadIdx.x, k_in = tid % kProjRows, c_in = tid / kProjRows;
+        constexpr int kColStep = kProjThreads / kProjRows;
+        N sum(0.0);
+        for (int base = 0; base < n; base += kProjRows) {
+            const int k = base + k_in;
+            const bool in = k < n && in_piston(st[k]);
+            const N w = in ? N(w_tab[k / M]) : N(0.0);
+            for (int c = c_in; c < P; c += kColStep)
+                term[c * kProjLd + k_in] = in ? value_of(w * N(col0[c * ap.rows + k])) : 0.0;
+            if (c_in == 0) term[P * kProjLd + k_in] = value_of(w);
+            __syncthreads();
+            if (tid <= P) {
+                const int rows = n - base < kProjRows ? n - base : kProjRows;
+                const double* t = term + tid * kProjLd;
+                for (int i = 0; i < rows; ++i) sum += N(t[i]);
+            }
+            __syncthreads();
         }
+        if (tid <= P) sums[tid] = value_of(sum);
         __syncthreads();
-    }
-    if (tid <= P) sums[tid] = value_of(sum);
-    __syncthreads();
-    const N w_ok = sums[P];
-    const bool valid = value_of(w_ok) > 0.0;
-    if (tid < P) sums[tid] = valid ? value_of(N(sums[tid]) / w_ok) : 0.0;
-    __syncthreads();
-    const N scale = p.scale[tu];
-    for (int k = k_in; k < n; k += kProjRows) {
-        const bool in = valid && in_piston(st[k]);
-        const N factor = scale * N(rw_tab[k / M]);
-        for (int c = c_in; c < P; c += kColStep) {
-            double* y = col0 + c * ap.rows + k;
-            *y = in ? value_of(factor * (N(*y) - N(sums[c]))) : 0.0;
+        const N w_ok = sums[P];
+        const bool valid = value_of(w_ok) > 0.0;
+        if (tid < P) sums[tid] = valid ? value_of(N(sums[tid]) / w_ok) : 0.0;
+        __syncthreads();
+        const N scale = p.scale[tu];
+        for (int k = k_in; k < n; k += kProjRows) {
+            const bool in = valid && in_piston(st[k]);
+            const N factor = scale * N(rw_tab[k / M]);
+            for (int c = c_in; c < P; c += kColStep) {
+                double* y = col0 + c * ap.rows + k;
+                *y = in ? value_of(factor * (N(*y) - N(sums[c]))) : 0.0;
+            }
         }
-    }
-    __syncthreads();  // the means are consumed
+        __syncthreads();  // the means are consumed
     }
 }
 
@@ -533,19 +533,19 @@ namespace mkb {
 // counter per run, no CTA waits) adds them up.
 namespace {
 
-// One CTA of 256 threads (FP64: 242 to 255 registers, nothing spilled without plates, transforms,
-// glass and stop, else at most 136 bytes of stores) or two (MIXED, FP32_BULK: 128 registers) per SM;
-// in plans of few rays (fused_threads) CTAs of 128 threads, three (FP64: 168 registers) or four. In
-// larger CTAs the warps of a scheduler are in the same phase more often and share its instruction
-// fetches (ncu: a quarter of the stalls of 128-thread CTAs were missing instructions), and one
-// accumulator and record serve twice the rays. 128 -> 256 threads: 512 objectives (FP64) 9.62 ->
-// 9.33 ms, 2,048 uneven systems (MIXED) 21.9 -> 19.9 ms, merit and gradient of 1,024 toleranced
-// samples 17.8 -> 17.0 ms, six LM iterations of 512 uneven systems (FP64_FMA) 53.5 -> 50.2 ms. 384
-// threads of 168 registers: 10.8 ms where 128 threads took 11.0 (FP64), 24.2 where they took 21.9
-// (MIXED).
-// Two MIXED CTAs fit an SM's shared memory up to 63 variables (64 surfaces of 7 wavelengths too); at
-// 64 from 20 surfaces of 7 wavelengths on it is one: 1,024 uneven systems with a widest run of 63
-// variables 11.2 ms, of 64 15.9 ms.
+// One CTA of 256 threads (FP64: 244 to 255 registers, nothing spilled without plates, transforms,
+// glass and stop, else at most 136 bytes of stores) or two (MIXED, FP32_BULK: 128 registers) per
+// SM; in plans of few rays (fused_threads) CTAs of 128 threads, three (FP64: 168 registers) or
+// four. In larger CTAs the warps of a scheduler are in the same phase more often and share its
+// instruction fetches (ncu: a quarter of the stalls of 128-thread CTAs were missing instructions),
+// and one accumulator and record serve twice the rays. 128 -> 256 threads: 512 objectives (FP64)
+// 9.62 -> 9.33 ms, 2,048 uneven systems (MIXED) 21.9 -> 19.9 ms, merit and gradient of 1,024
+// toleranced samples 17.8 -> 17.0 ms, six LM iterations of 512 uneven systems (FP64_FMA) 53.5 ->
+// 50.2 ms. 384 threads of 168 registers: 10.8 ms where 128 threads took 11.0 (FP64), 24.2 where
+// they took 21.9 (MIXED).
+// Two MIXED CTAs fit an SM's shared memory up to 63 variables (64 surfaces of 7 wavelengths too);
+// at 64 from 20 surfaces of 7 wavelengths on it is one: 1,024 uneven systems with a widest run of
+// 63 variables 11.2 ms, of 64 15.9 ms.
 constexpr int kFusedThreads = 256, kFusedThreadsSmall = 128;
 constexpr int kSmallPlanRays = 3072;  // most rays of a run that takes the small block
 // CTAs per SM that the registers are budgeted for
@@ -1088,18 +1088,18 @@ int groups_of(int pieces) { return pieces < kPieceGroups ? pieces : kPieceGroups
 // systems of 648 rays 900 -> 620 / 520 -> 420, 16,384 of 15 rays 1,780 -> 690 / 880 -> 480, 2,048
 // systems of 20 surfaces and 2,520 rays 6,150 -> 4,740 / 3,420 -> 2,970. From 3,640 rays on glass
 // variables (2,840 -> 3,100 / 1,500 -> 1,630) and tilted systems of 21 surfaces lose by it. Below,
-// the widest runs do: 4,096 of P = 61 and 150 rays 2,220 -> 2,640 / 1,270 -> 1,520, where one CTA of
-// two waves stands for two.
+// the widest runs do: 4,096 of P = 61 and 150 rays 2,220 -> 2,570 / 1,270 -> 1,520, two blocks of
+// 128 where one of 256 would do and two CTAs to an SM.
 int fused_threads(const TraceParams& p) {
     return p.rays <= kSmallPlanRays ? kFusedThreadsSmall : kFusedThreads;
 }
 
 // Pieces of whole tuples and of at least two blocks of rays, more when a run would otherwise have
 // more than kMaxPieces. In plans of few rays a block left mostly idle is a large part of the run:
-// pieces are one and a half to four blocks there, none is shorter, and of the ends in that range the
-// first is taken that leaves at most 1/16 of its blocks' threads idle, else the one that leaves the
-// fewest (4,096 systems of 15 tuples of 48 rays, FP64: 2,230 us with the first end of two blocks,
-// 2,010 us so).
+// pieces are one and a half to four blocks there, none is shorter, and of the ends in that range
+// the first is taken that leaves at most 1/16 of its blocks' threads idle, else the one that
+// leaves the fewest (4,096 systems of 15 tuples of 48 rays, FP64: 2,230 us with the first end of
+// two blocks, 2,010 us so).
 FusedPieces make_pieces(const TraceParams& p) {
     FusedPieces c{};
     const int block = fused_threads(p), least = (p.rays + kMaxPieces - 1) / kMaxPieces;
@@ -1188,7 +1188,7 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
     YT* Y = reinterpret_cast<YT*>(mu_tab + (((p.S + 1) * p.L + 1) & ~1));  // [NPM][TS]
     double* R = reinterpret_cast<double*>(Y + NPM * TS);  // [TS] the residual column
     double* E = R + TS;                                // column-major [NPM][kExtraStride]
-    double* mu_open = E + NPM * kExtraStride;                    // [NPM] running mean of the open tuple
+    double* mu_open = E + NPM * kExtraStride;          // [NPM] running mean of the open tuple
     double* seg_mean = mu_open + NPM;                  // [kSegBatch][NPM] segment means
     double* seg_w = seg_mean + kSegBatch * NPM;        // [kSegBatch] segment weights
     double* acc = seg_w + kSegBatch;                   // [pairs][32][2] DMMA accumulators
@@ -1258,219 +1258,226 @@ adjoint_gram_kernel(const __grid_constant__ FusedArgs fa) {
                 aim_sensitivity(record, lay, v, k, aim_sens[k], aim_sens[MKB_MAX_VARIABLES + k]);
         __syncthreads();
         for (int piece = piece0; piece < piece1; ++piece) {
-        const int piece_end = fa.pc.ray[piece + 1];
-        // the open tuple (kept identically by every thread): its index and weight
-        int open_tuple = -1;
-        bool extra = false;  // the chunk has an extra row
-        double open_w = 0.0;
-        for (int i = tid; i < pairs * 64; i += kT) acc[i] = 0.0;
-        for (int base = fa.pc.ray[piece]; base < piece_end; base += kT) {
-            const int q = base + tid;
-            YT* row = Y + tid;  // this ray's row, column c at row[c * TS]
-            for (int c = 0; c < NP; ++c) row[c * TS] = YT(0);
-            YT* prow = pen_slot + tid;  // this ray's penalty row, column c at prow[c * T]
-            int tu = -1, status = kMissed;
-            bool has_pen = false;
-            double pen_val = 0.0, opl_val = 0.0;
-            Sample smp{};
-            if (q < piece_end) {
-                int f = 0;
-                while (f + 1 < p.F && q >= p.field_offset[f + 1]) ++f;
-                const int within = q - p.field_offset[f];
-                const int l = within / p.sample_count[f];
-                const int k = within - l * p.sample_count[f];
-                tu = f * p.L + l;
-                smp = pupil_sample(p, sh.tab, f, k);
-                int soft_first = kOk, count = 0, image_branch = 0;
-                uint64_t br_lo = 0, br_hi = 0;
-                double opl = 0.0, penalty = 0.0;
-                if constexpr (std::is_same<N, BulkPrecision>::value)
-                    fused_forward_bulk<Keep, kT>(p, record, mu_tab, lay, S, f, l, smp, soft_mode,
-                                             my_ck, stride_ck, br_lo, br_hi, count,
-                                             image_branch, status, soft_first, opl, penalty);
-                else
-                    fused_forward<typename FusedTypes<N>::Fwd, Keep, kFeat, kT>(
-                        p, record, mu_tab, lay, S, f, l, smp, soft_mode, my_ck, stride_ck, br_lo,
-                        br_hi, count, image_branch, status, soft_first, opl, penalty);
-                const bool piston = in_piston(status);
-                has_pen = soft_mode && status != kOk;
-                const bool pen_sweep = has_pen && soft_first != kOk;
-                const double pfac = has_pen ? p.pscale[tu] * smp.root_weight : 0.0;
-                if (has_pen) {
-                    for (int c = 0; c < NP; ++c) prow[c * kT] = YT(0);
-                    pen_val = pfac * (is_soft(status) ? penalty : penalty + 1.0);
-                }
-                if (piston) opl_val = opl;
-                // the OPL row into Y, the penalty row into the scratch slot
-                if (kFusedDual && __any_sync(__activemask(), piston && pen_sweep)) {
-                    if (piston || pen_sweep) {
-                        const double so[2] = {piston ? 1.0 : 0.0, 0.0};
-                        const double sp[2] = {0.0, pen_sweep ? 1.0 : 0.0};
-                        const RowSinks<2, YT> sinks{{1.0, pfac}, {row, prow}, {TS, kT}};
-                        run_backward<N, 2, kFeat, kT, ReciprocalDivisor>(
-                            p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
-                            count, image_branch, piston, soft_mode, so, sp, sinks, aim_sens);
+            const int piece_end = fa.pc.ray[piece + 1];
+            // the open tuple (kept identically by every thread): its index and weight
+            int open_tuple = -1;
+            bool extra = false;  // the chunk has an extra row
+            double open_w = 0.0;
+            for (int i = tid; i < pairs * 64; i += kT) acc[i] = 0.0;
+            for (int base = fa.pc.ray[piece]; base < piece_end; base += kT) {
+                const int q = base + tid;
+                YT* row = Y + tid;  // this ray's row, column c at row[c * TS]
+                for (int c = 0; c < NP; ++c) row[c * TS] = YT(0);
+                YT* prow = pen_slot + tid;  // this ray's penalty row, column c at prow[c * T]
+                int tu = -1, status = kMissed;
+                bool has_pen = false;
+                double pen_val = 0.0, opl_val = 0.0;
+                Sample smp{};
+                if (q < piece_end) {
+                    int f = 0;
+                    while (f + 1 < p.F && q >= p.field_offset[f + 1]) ++f;
+                    const int within = q - p.field_offset[f];
+                    const int l = within / p.sample_count[f];
+                    const int k = within - l * p.sample_count[f];
+                    tu = f * p.L + l;
+                    smp = pupil_sample(p, sh.tab, f, k);
+                    int soft_first = kOk, count = 0, image_branch = 0;
+                    uint64_t br_lo = 0, br_hi = 0;
+                    double opl = 0.0, penalty = 0.0;
+                    if constexpr (std::is_same<N, BulkPrecision>::value)
+                        fused_forward_bulk<Keep, kT>(p, record, mu_tab, lay, S, f, l, smp,
+                                                     soft_mode, my_ck, stride_ck, br_lo, br_hi,
+                                                     count, image_branch, status, soft_first, opl,
+                                                     penalty);
+                    else
+                        fused_forward<typename FusedTypes<N>::Fwd, Keep, kFeat, kT>(
+                            p, record, mu_tab, lay, S, f, l, smp, soft_mode, my_ck, stride_ck,
+                            br_lo, br_hi, count, image_branch, status, soft_first, opl, penalty);
+                    const bool piston = in_piston(status);
+                    has_pen = soft_mode && status != kOk;
+                    const bool pen_sweep = has_pen && soft_first != kOk;
+                    const double pfac = has_pen ? p.pscale[tu] * smp.root_weight : 0.0;
+                    if (has_pen) {
+                        for (int c = 0; c < NP; ++c) prow[c * kT] = YT(0);
+                        pen_val = pfac * (is_soft(status) ? penalty : penalty + 1.0);
                     }
-                } else if (!(piston && pen_sweep)) {
-                    if (piston || pen_sweep) {  // one row: its seed and its sink
-                        const double so[1] = {piston ? 1.0 : 0.0};
-                        const double sp[1] = {pen_sweep ? 1.0 : 0.0};
-                        const RowSinks<1, YT> sinks{{piston ? 1.0 : pfac}, {piston ? row : prow},
-                                                {piston ? TS : kT}};
+                    if (piston) opl_val = opl;
+                    // the OPL row into Y, the penalty row into the scratch slot
+                    if (kFusedDual && __any_sync(__activemask(), piston && pen_sweep)) {
+                        if (piston || pen_sweep) {
+                            const double so[2] = {piston ? 1.0 : 0.0, 0.0};
+                            const double sp[2] = {0.0, pen_sweep ? 1.0 : 0.0};
+                            const RowSinks<2, YT> sinks{{1.0, pfac}, {row, prow}, {TS, kT}};
+                            run_backward<N, 2, kFeat, kT, ReciprocalDivisor>(
+                                p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
+                                br_hi, count, image_branch, piston, soft_mode, so, sp, sinks,
+                                aim_sens);
+                        }
+                    } else if (!(piston && pen_sweep)) {
+                        if (piston || pen_sweep) {  // one row: its seed and its sink
+                            const double so[1] = {piston ? 1.0 : 0.0};
+                            const double sp[1] = {pen_sweep ? 1.0 : 0.0};
+                            const RowSinks<1, YT> sinks{{piston ? 1.0 : pfac},
+                                                        {piston ? row : prow},
+                                                        {piston ? TS : kT}};
+                            run_backward<N, 1, kFeat, kT, ReciprocalDivisor>(
+                                p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
+                                br_hi, count, image_branch, piston, soft_mode, so, sp, sinks,
+                                aim_sens);
+                        }
+                    } else {  // both rows, one sweep each
+                        const double so0[1] = {1.0}, sp0[1] = {0.0};
+                        const RowSinks<1, YT> s0{{1.0}, {row}, {TS}};
                         run_backward<N, 1, kFeat, kT, ReciprocalDivisor>(
-                            p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
-                            count, image_branch, piston, soft_mode, so, sp, sinks, aim_sens);
+                                p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
+                                br_hi, count, image_branch, true, soft_mode, so0, sp0, s0,
+                                aim_sens);
+                        const double so1[1] = {0.0}, sp1[1] = {1.0};
+                        const RowSinks<1, YT> s1{{pfac}, {prow}, {kT}};
+                        run_backward<N, 1, kFeat, kT, ReciprocalDivisor>(
+                                p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo,
+                                br_hi, count, image_branch, true, soft_mode, so1, sp1, s1,
+                                aim_sens);
                     }
-                } else {  // both rows, one sweep each
-                    const double so0[1] = {1.0}, sp0[1] = {0.0};
-                    const RowSinks<1, YT> s0{{1.0}, {row}, {TS}};
-                    run_backward<N, 1, kFeat, kT, ReciprocalDivisor>(
-                            p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
-                            count, image_branch, true, soft_mode, so0, sp0, s0, aim_sens);
-                    const double so1[1] = {0.0}, sp1[1] = {1.0};
-                    const RowSinks<1, YT> s1{{pfac}, {prow}, {kT}};
-                    run_backward<N, 1, kFeat, kT, ReciprocalDivisor>(
-                            p, v, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi,
-                            count, image_branch, true, soft_mode, so1, sp1, s1, aim_sens);
                 }
-            }
-            R[tid] = opl_val;
-            const double wv = (q < piece_end && in_piston(status)) ? smp.weight : 0.0;
-            const double swv = sqrt(wv);
-            sh.w[tid] = wv;
-            if (tid == 0) sh.any_pen = 0;
-            __syncthreads();
-            if (has_pen) sh.any_pen = 1;
-            // ---- B: centre every tuple segment of the chunk ----
-            const int rows_here = piece_end - base < kT ? piece_end - base : kT;
-            // Segments are the chunk's pieces of its tuples; rays are ordered by tuple (f-major,
-            // then l), so segment k is tuple t0 + k and its rows follow from the plan alone.
-            const int t0 = tuple_of(p, base);
-            const int nseg = tuple_of(p, base + rows_here - 1) - t0 + 1;
-            const int seg = tid < rows_here ? tu - t0 : -1;
-            auto seg_rows = [&](int k, int& a, int& n) {
-                const int t = t0 + k;
-                const int f = t / p.L;
-                const int start = p.field_offset[f] + (t - f * p.L) * p.sample_count[f] - base;
-                a = start > 0 ? start : 0;
-                const int end = start + p.sample_count[f];
-                n = (end < rows_here ? end : rows_here) - a;
-                if (n < 0) n = 0;
-            };
-            for (int k0 = 0; k0 < nseg; k0 += kSegBatch) {
-                const int kn = nseg - k0 < kSegBatch ? nseg - k0 : kSegBatch;
-                // B2: weight and weighted column means of each segment, eight lanes per (segment,
-                // two columns) taking rows h, h + 8, ... (h = lane mod 8) and a three-step
-                // shuffle sum; two columns share the weights' loads and their sum. The lanes of
-                // a (half-)warp hit different banks (column stride 4 mod 32 floats, 4 mod 16
-                // doubles).
-                {
-                    const int h = lane & 7;
-                    const unsigned octet = 0xFFu << (lane & ~7);
-                    const int halves = (P >> 1) + 1;  // column pairs of 0 .. P
-                    for (int pr = tid >> 3; pr < kn * halves; pr += kT / 8) {
-                        const int k = pr / halves, c0 = 2 * (pr - k * halves);
-                        const int c1 = c0 < P ? c0 + 1 : P;
-                        int a, n;
-                        seg_rows(k0 + k, a, n);
-                        const YT* col0 = Y + c0 * TS + a;
-                        const YT* col1 = Y + c1 * TS + a;
-                        const double* rcol = R + a;
-                        const double* wr = sh.w + a;
-                        const bool r0 = c0 == P, r1 = c1 == P;  // the residual column
-                        double sw_sum = 0.0, sum0 = 0.0, sum1 = 0.0;
+                R[tid] = opl_val;
+                const double wv = (q < piece_end && in_piston(status)) ? smp.weight : 0.0;
+                const double swv = sqrt(wv);
+                sh.w[tid] = wv;
+                if (tid == 0) sh.any_pen = 0;
+                __syncthreads();
+                if (has_pen) sh.any_pen = 1;
+                // ---- B: centre every tuple segment of the chunk ----
+                const int rows_here = piece_end - base < kT ? piece_end - base : kT;
+                // Segments are the chunk's pieces of its tuples; rays are ordered by tuple
+                // (f-major, then l), so segment k is tuple t0 + k and its rows follow from the
+                // plan alone.
+                const int t0 = tuple_of(p, base);
+                const int nseg = tuple_of(p, base + rows_here - 1) - t0 + 1;
+                const int seg = tid < rows_here ? tu - t0 : -1;
+                auto seg_rows = [&](int k, int& a, int& n) {
+                    const int t = t0 + k;
+                    const int f = t / p.L;
+                    const int start = p.field_offset[f] + (t - f * p.L) * p.sample_count[f] - base;
+                    a = start > 0 ? start : 0;
+                    const int end = start + p.sample_count[f];
+                    n = (end < rows_here ? end : rows_here) - a;
+                    if (n < 0) n = 0;
+                };
+                for (int k0 = 0; k0 < nseg; k0 += kSegBatch) {
+                    const int kn = nseg - k0 < kSegBatch ? nseg - k0 : kSegBatch;
+                    // B2: weight and weighted column means of each segment, eight lanes per
+                    // (segment, two columns) taking rows h, h + 8, ... (h = lane mod 8) and a
+                    // three-step shuffle sum; two columns share the weights' loads and their sum.
+                    // The lanes of a (half-)warp hit different banks (column stride 4 mod 32
+                    // floats, 4 mod 16 doubles).
+                    {
+                        const int h = lane & 7;
+                        const unsigned octet = 0xFFu << (lane & ~7);
+                        const int halves = (P >> 1) + 1;  // column pairs of 0 .. P
+                        for (int pr = tid >> 3; pr < kn * halves; pr += kT / 8) {
+                            const int k = pr / halves, c0 = 2 * (pr - k * halves);
+                            const int c1 = c0 < P ? c0 + 1 : P;
+                            int a, n;
+                            seg_rows(k0 + k, a, n);
+                            const YT* col0 = Y + c0 * TS + a;
+                            const YT* col1 = Y + c1 * TS + a;
+                            const double* rcol = R + a;
+                            const double* wr = sh.w + a;
+                            const bool r0 = c0 == P, r1 = c1 == P;  // the residual column
+                            double sw_sum = 0.0, sum0 = 0.0, sum1 = 0.0;
 #pragma unroll 4
-                        for (int r = h; r < n; r += 8) {
-                            const double w = wr[r];
-                            sw_sum += w;
-                            sum0 += w * (r0 ? rcol[r] : static_cast<double>(col0[r]));
-                            sum1 += w * (r1 ? rcol[r] : static_cast<double>(col1[r]));
-                        }
+                            for (int r = h; r < n; r += 8) {
+                                const double w = wr[r];
+                                sw_sum += w;
+                                sum0 += w * (r0 ? rcol[r] : static_cast<double>(col0[r]));
+                                sum1 += w * (r1 ? rcol[r] : static_cast<double>(col1[r]));
+                            }
 #pragma unroll
-                        for (int o = 1; o <= 4; o <<= 1) {
-                            sw_sum += __shfl_xor_sync(octet, sw_sum, o);
-                            sum0 += __shfl_xor_sync(octet, sum0, o);
-                            sum1 += __shfl_xor_sync(octet, sum1, o);
-                        }
-                        if (h < 2) {
-                            const double sum = h == 0 ? sum0 : sum1;
-                            seg_mean[k * NP + (h == 0 ? c0 : c1)] =
-                                sw_sum > 0.0 ? sum / sw_sum : 0.0;
-                            if (h == 0 && c0 == 0) seg_w[k] = sw_sum;
+                            for (int o = 1; o <= 4; o <<= 1) {
+                                sw_sum += __shfl_xor_sync(octet, sw_sum, o);
+                                sum0 += __shfl_xor_sync(octet, sum0, o);
+                                sum1 += __shfl_xor_sync(octet, sum1, o);
+                            }
+                            if (h < 2) {
+                                const double sum = h == 0 ? sum0 : sum1;
+                                seg_mean[k * NP + (h == 0 ? c0 : c1)] =
+                                    sw_sum > 0.0 ? sum / sw_sum : 0.0;
+                                if (h == 0 && c0 == 0) seg_w[k] = sw_sum;
+                            }
                         }
                     }
-                }
-                __syncthreads();
-                // B3: every row of the batch's segments centred and scaled by its own thread
-                if (seg >= k0 && seg < k0 + kn) {
-                    const int k = seg - k0;
-                    const double f = (seg_w[k] > 0.0 && wv > 0.0) ? p.scale[tu] * swv : 0.0;
-                    const double* m = seg_mean + k * NP;
-                    for (int c = 0; c < P; ++c) {
-                        YT* y = Y + c * TS + tid;
-                        *y = f != 0.0 ? YT(f * (static_cast<double>(*y) - m[c])) : YT(0);
+                    __syncthreads();
+                    // B3: every row of the batch's segments centred and scaled by its own thread
+                    if (seg >= k0 && seg < k0 + kn) {
+                        const int k = seg - k0;
+                        const double f = (seg_w[k] > 0.0 && wv > 0.0) ? p.scale[tu] * swv : 0.0;
+                        const double* m = seg_mean + k * NP;
+                        for (int c = 0; c < P; ++c) {
+                            YT* y = Y + c * TS + tid;
+                            *y = f != 0.0 ? YT(f * (static_cast<double>(*y) - m[c])) : YT(0);
+                        }
+                        R[tid] = f != 0.0 ? f * (R[tid] - m[P]) : 0.0;
                     }
-                    R[tid] = f != 0.0 ? f * (R[tid] - m[P]) : 0.0;
-                }
-                // B4: the segments merged into the open tuple in row order (threads = columns
-                // for the vectors; the scalar state is updated identically by every thread).
-                // Only the chunk's first segment can go on with an open tuple: one extra row.
-                for (int k = 0; k < kn; ++k) {
-                    const double ws = seg_w[k];
-                    if (!(ws > 0.0)) continue;
-                    const int t = t0 + k0 + k;
-                    const bool open = open_tuple == t && open_w > 0.0;
-                    if (tid <= P) {
-                        const double mean = seg_mean[k * NP + tid];
+                    // B4: the segments merged into the open tuple in row order (threads = columns
+                    // for the vectors; the scalar state is updated identically by every thread).
+                    // Only the chunk's first segment can go on with an open tuple: one extra row.
+                    for (int k = 0; k < kn; ++k) {
+                        const double ws = seg_w[k];
+                        if (!(ws > 0.0)) continue;
+                        const int t = t0 + k0 + k;
+                        const bool open = open_tuple == t && open_w > 0.0;
+                        if (tid <= P) {
+                            const double mean = seg_mean[k * NP + tid];
+                            if (open) {
+                                const double fac = p.scale[t] * sqrt(open_w * ws / (open_w + ws));
+                                E[tid * kExtraStride] = fac * (mean - mu_open[tid]);
+                                mu_open[tid] += (ws / (open_w + ws)) * (mean - mu_open[tid]);
+                            } else {
+                                mu_open[tid] = mean;
+                            }
+                        }
                         if (open) {
-                            const double fac = p.scale[t] * sqrt(open_w * ws / (open_w + ws));
-                            E[tid * kExtraStride] = fac * (mean - mu_open[tid]);
-                            mu_open[tid] += (ws / (open_w + ws)) * (mean - mu_open[tid]);
+                            extra = true;
+                            open_w += ws;
                         } else {
-                            mu_open[tid] = mean;
+                            open_tuple = t;
+                            open_w = ws;
                         }
                     }
-                    if (open) {
-                        extra = true;
-                        open_w += ws;
-                    } else {
-                        open_tuple = t;
-                        open_w = ws;
-                    }
+                    __syncthreads();
                 }
-                __syncthreads();
-            }
-            // ---- C: the centred rows and the extra row ----
-            accumulate_rows<kT>(Y, R, TS, P, (rows_here + 3) & ~3, pairs, sh.tiles, acc);
-            if (extra) accumulate<kT>(E, kExtraStride, 4, pairs, sh.tiles, acc);
-            __syncthreads();
-            extra = false;
-            // ---- D: penalty rows ----
-            if (sh.any_pen) {
-                for (int c = 0; c < NP; ++c) row[c * TS] = has_pen ? prow[c * kT] : YT(0);
-                R[tid] = pen_val;
-                __syncthreads();
+                // ---- C: the centred rows and the extra row ----
                 accumulate_rows<kT>(Y, R, TS, P, (rows_here + 3) & ~3, pairs, sh.tiles, acc);
+                if (extra) accumulate<kT>(E, kExtraStride, 4, pairs, sh.tiles, acc);
                 __syncthreads();
+                extra = false;
+                // ---- D: penalty rows ----
+                if (sh.any_pen) {
+                    for (int c = 0; c < NP; ++c) row[c * TS] = has_pen ? prow[c * kT] : YT(0);
+                    R[tid] = pen_val;
+                    __syncthreads();
+                    accumulate_rows<kT>(Y, R, TS, P, (rows_here + 3) & ~3, pairs, sh.tiles, acc);
+                    __syncthreads();
+                }
             }
-        }
-        // ---- the piece's sum into its group's, the group's into the run's (every element by
-        // the thread that owns it) ----
-        if (fa.items == fa.pc.count && fa.items > 1) continue;
-        int g = 0;
-        while (piece >= fa.pc.first[g + 1]) ++g;
-        const bool opens = piece == fa.pc.first[g], closes = piece + 1 == fa.pc.first[g + 1];
-        for (int i = tid; i < pairs * 64; i += kT) {
-            double s = acc[i];
-            if (!opens) s = group_sum[i] + s;
-            if (!closes) {
-                group_sum[i] = s;
-            } else {
-                if (g > 0 && fa.items == 1) s = run_sum[i] + s;
-                if (fa.items == 1 && g + 1 < fa.pc.groups) run_sum[i] = s;
-                acc[i] = s;
+            // ---- the piece's sum into its group's, the group's into the run's (every element by
+            // the thread that owns it) ----
+            if (fa.items == fa.pc.count && fa.items > 1) continue;
+            int g = 0;
+            while (piece >= fa.pc.first[g + 1]) ++g;
+            const bool opens = piece == fa.pc.first[g], closes = piece + 1 == fa.pc.first[g + 1];
+            for (int i = tid; i < pairs * 64; i += kT) {
+                double s = acc[i];
+                if (!opens) s = group_sum[i] + s;
+                if (!closes) {
+                    group_sum[i] = s;
+                } else {
+                    if (g > 0 && fa.items == 1) s = run_sum[i] + s;
+                    if (fa.items == 1 && g + 1 < fa.pc.groups) run_sum[i] = s;
+                    acc[i] = s;
+                }
             }
-        }
         }
         if (fa.items > 1) {
             // leave the item's sum; the CTA that brings the run's last adds them up
@@ -1579,9 +1586,9 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
         int status, soft_first = kOk, count = 0, image_branch = 0;
         uint64_t br_lo = 0, br_hi = 0;
         double opl, penalty;
-        fused_forward<N, double, kFeat, kRowsThreads>(p, record, mu_tab, lay, S, f, l, smp, soft_mode,
-                                                      my_ck, stride_ck, br_lo, br_hi, count,
-                                                      image_branch, status, soft_first, opl,
+        fused_forward<N, double, kFeat, kRowsThreads>(p, record, mu_tab, lay, S, f, l, smp,
+                                                      soft_mode, my_ck, stride_ck, br_lo, br_hi,
+                                                      count, image_branch, status, soft_first, opl,
                                                       penalty);
         const bool piston = in_piston(status);
         const bool pen = soft_mode && soft_first != kOk;
@@ -1598,17 +1605,17 @@ kept_rows_kernel(const __grid_constant__ RowsArgs ra) {
                 {1.0, pfac},
                 {piston ? row : unused, pen ? row + p.rays : unused},
                 {piston ? ra.ap.rows : 0, pen ? ra.ap.rows : 0}};
-            run_backward<N, 2, kFeat, kRowsThreads, Divisor>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
-                                      br_lo, br_hi, count, image_branch, piston, soft_mode, so, sp,
-                                      sinks, nullptr);
+            run_backward<N, 2, kFeat, kRowsThreads, Divisor>(
+                p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi, count,
+                image_branch, piston, soft_mode, so, sp, sinks, nullptr);
         } else {
             const double so[1] = {piston ? 1.0 : 0.0};
             const double sp[1] = {pen ? 1.0 : 0.0};
             const RowSinks<1, double, int64_t> sinks{
                 {piston ? 1.0 : pfac}, {piston ? row : row + p.rays}, {ra.ap.rows}};
-            run_backward<N, 1, kFeat, kRowsThreads, Divisor>(p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck,
-                                      br_lo, br_hi, count, image_branch, piston, soft_mode, so, sp,
-                                      sinks, nullptr);
+            run_backward<N, 1, kFeat, kRowsThreads, Divisor>(
+                p, vars, record, mu_tab, lay, S, f, l, smp, my_ck, stride_ck, br_lo, br_hi, count,
+                image_branch, piston, soft_mode, so, sp, sinks, nullptr);
         }
     }
 }
@@ -1652,8 +1659,9 @@ int launch_adjoint_rows(const TraceParams& tp, const VarParams& vp, int64_t rows
         set_error("adjoint rows: scratch of %zu bytes needed", adjoint_rows_scratch_bytes(tp));
         return MKB_ERR_WORKSPACE;
     }
-    auto kernel = exact ? (vp.has_glass ? kept_rows_kernel<Exact64, 4> : kept_rows_kernel<Exact64, 0>)
-                        : (vp.has_glass ? kept_rows_kernel<double, 4> : kept_rows_kernel<double, 0>);
+    const bool glass = vp.has_glass != 0;
+    auto kernel = exact ? (glass ? kept_rows_kernel<Exact64, 4> : kept_rows_kernel<Exact64, 0>)
+                        : (glass ? kept_rows_kernel<double, 4> : kept_rows_kernel<double, 0>);
     const size_t smem = sizeof(double) * (static_cast<size_t>((tp.stride + 1) & ~1) +
                                           static_cast<size_t>((tp.S + 1) * tp.L));
     int dev = 0, sms = 0, per_sm = 0;

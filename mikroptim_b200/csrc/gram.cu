@@ -205,8 +205,8 @@ __device__ inline void dmma_8x8x4(double& d0, double& d1, double a, double b) {
 // same entries (lane l: column l / 4, row l % 4), so every warp streams its own rows straight from
 // memory, 32 bytes of each column at a time, and the eight warps' sums are added in order. The
 // tiles below leave seven warps idle here and wait for a tile at a time; 1,024 runs of P = 4 and
-// 900 rows, in L2: 32.5 us there, 6.7 us here. Which way a run goes is decided by its own P alone, so
-// that its bits are the same in every batch. part: [kDmmaWarps * 64] in shared memory.
+// 900 rows, in L2: 32.5 us there, 6.7 us here. Which way a run goes is decided by its own P alone,
+// so that its bits are the same in every batch. part: [kDmmaWarps * 64] in shared memory.
 __device__ __forceinline__ void one_tile_sums(const double* J, const double* r, int64_t run, int P,
                                               int stride, int64_t R, double* part, double* gram) {
     const int n = P + 1;

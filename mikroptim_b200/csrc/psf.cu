@@ -6,7 +6,8 @@
 // (PsfEngine::compute, src/cuda/psf.cu; CPU reference psf_cpu, src/eval/psf.cpp:330). Here the
 // transform is this file's own shared-memory FFT, built around the zero padding:
 //   psf_rows_kernel     the N non-zero rows of every pupil field: exp(i phase) of the row's N
-//                       points, a length-M FFT in shared memory, the row spectra to HBM
+//                       points, formed by the first pass of a length-M FFT in shared memory, the
+//                       row spectra to HBM
 //                       column-major ([T][M][N] complex; the M - N zero rows are never
 //                       formed)
 //   psf_cols_kernel     C adjacent columns per CTA: the N non-zero entries of each column, a
@@ -14,10 +15,9 @@
 //                       centred PSF written once, and the two projections of I the MTF cuts
 //                       need: per column the sum over the rows (in a fixed order), per row the
 //                       sum over this CTA's columns (a partial per tile)
-//   psf_mtf_kernel      per tuple: OTF(k, 0) and OTF(0, k), k = 0 .. N, as direct DFTs of the
-//                       two projections (OTF(kx, 0) = sum_q colsum[q] exp(+2 pi i kx q / M)),
-//                       OTF(0) = sum of the column sums; a warp per frequency, fixed-order
-//                       shuffle sums -- no inverse 2-D transform
+//   psf_mtf_kernel      per tuple: OTF(k, 0) and OTF(0, k), k = 0 .. N, from one length-M FFT of
+//                       (column sums) + i (row sums), both real (OTF(kx, 0) = sum_q colsum[q]
+//                       exp(+2 pi i kx q / M)); OTF(0) is its element 0 -- no inverse 2-D transform
 // Everything is FP64; every sum has a fixed order, so results repeat bit for bit. Against the
 // reference's radix-2 CPU FFT the PSF and MTF agree to rounding (the reference's own CPU/GPU bar
 // is 1e-13 in units of the unaberrated peak, tests/tolerances.hpp:286).

@@ -16,9 +16,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision", [PRECISION_FP64, PRECISION_FP64_FMA, PRECISION_MIXED])
 @pytest.mark.parametrize("variants,rings,spokes", [
-    (3, 1, 1),      # 35 rays: one piece, a chunk of 35 rows
+    (3, 1, 1),      # 35 rays: one piece, a chunk of 35 rows on a block of 128
     (2, 8, 16),     # 9 pieces, an item each
-    (1200, 8, 16),  # four groups
+    (1200, 8, 16),  # one item per run (FP64), four groups (MIXED)
     (4200, 8, 16),  # one item per run
     (5, 7, 19),     # 133 rays per tuple: chunks that end inside a tuple
     (1, 32, 64),    # 35 pieces of 2,048 rays

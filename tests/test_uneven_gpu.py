@@ -118,9 +118,8 @@ def _gram_errors(ref, got):
 def test_uneven_mixed_fused_normal_equations_both_launches_against_fp64():
     """The headline kernel instance: the fused adjoint + normal equations in MIXED precision
     (FP64 trace, FP32 reverse sweep and FP32 derivative rows) on configuration-3 runs with full
-    16 x 32 pupils, through both of its launches -- runs with <= 31 variables, and the launch
-    sized for the widest run -- against the FP64 fused normal equations (separately rounded
-    operations, within 1e-10 of the exact ones). Bar per entry, relative to sqrt(A_ii A_jj):
+    16 x 32 pupils, the runs with <= 31 variables and the wider ones of one launch, against the
+    FP64 fused normal equations (separately rounded operations, within 1e-10 of the exact ones). Bar per entry, relative to sqrt(A_ii A_jj):
     median <= 1e-6 (narrow runs) and 1e-4 (wide runs: longer systems, 17 to 30 surfaces,
     accumulate more FP32 rounding in the sweep), every entry <= 2e-3. Measured on 256 runs:
     median 1.9e-7 / 2.5e-5, maximum 5.5e-4 / 7.1e-4."""
